@@ -23,9 +23,25 @@ void fill_prim(DPrim<R>& d, const smcrt_prim& s) {
     }
 }
 
+// The plain shape of a region (RegionShape): a single box, sphere or capsule
+// without modifiers whose rotation part is exactly the identity.
+int region_shape(const smcrt_scene* s, const smcrt_region& g) {
+    if (g.nprims != 1) return SHAPE_GENERIC;
+    const smcrt_prim& p = s->prims[g.first_prim];
+    if (p.nmods != 0) return SHAPE_GENERIC;
+    for (int i = 0; i < 3; ++i)
+        for (int j = 0; j < 3; ++j)
+            if (p.transform[i][j] != (i == j ? 1.0 : 0.0)) return SHAPE_GENERIC;
+    return p.kind == SMCRT_BOX       ? SHAPE_BOX
+           : p.kind == SMCRT_SPHERE  ? SHAPE_SPHERE
+           : p.kind == SMCRT_CAPSULE ? SHAPE_CAPSULE
+                                     : SHAPE_GENERIC;
+}
+
 template <class R>
-void fill_region(DRegion<R>& r, const smcrt_region& g) {
+void fill_region(DRegion<R>& r, const smcrt_scene* s, const smcrt_region& g) {
     std::memset(&r, 0, sizeof(r));
+    r.shape = region_shape(s, g);
     r.first = g.first_prim;
     r.n = g.nprims;
     r.op = g.op;
@@ -53,7 +69,7 @@ void fill_scene(SceneT<R>& d, const smcrt_scene* s) {
     d.nregions = s->nregions;
     d.nprims = s->nprims;
     for (int i = 0; i < s->nprims; ++i) fill_prim(d.prim[i], s->prims[i]);
-    for (int i = 0; i < s->nregions; ++i) fill_region(d.region[i], s->regions[i]);
+    for (int i = 0; i < s->nregions; ++i) fill_region(d.region[i], s, s->regions[i]);
 }
 
 // Bounding sphere of region r in world coordinates, for the sweep's cull
@@ -130,7 +146,7 @@ void scene_tables(const smcrt_scene* s, const smcrt_grid* grid, std::vector<DPri
     double scale = 1.0;
     if (grid) scale = std::fmax(scale, std::fmax(grid->xmax, std::fmax(grid->ymax, grid->zmax)));
     for (int i = 0; i < s->nregions; ++i) {
-        fill_region(regions[i], s->regions[i]);
+        fill_region(regions[i], s, s->regions[i]);
         double c[3], rad;
         if (region_bound(s, i, c, &rad)) {
             for (int a = 0; a < 3; ++a) bounds[4 * i + a] = (R)c[a];
@@ -223,9 +239,9 @@ __global__ void k_emit(const __grid_constant__ Params<R> P, long long first, lon
     emit(P, pk, rng);
     // the launch sweep as the transport kernel takes it: within near_band of a
     // surface, FP32 transport decides on the FP64 position with the FP64 scene
-    const SweepOut<R> o = sweep_regions<R, true>(P.sc, cv<R>(pk.pos), 0);
+    const SweepOut<R> o = sweep_regions<R, true>(P.sc, cv<R>(pk.pos), -1, true);
     int lay = o.lay;
-    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true>(P.sc64, pk.pos, 0).lay;
+    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true>(P.sc64, pk.pos, -1, true).lay;
     layer[i] = lay + 1;
     pos[3 * i] = pk.pos.x;
     pos[3 * i + 1] = pk.pos.y;

@@ -362,18 +362,17 @@ __device__ __forceinline__ void cache_move(Flight<R>& f) {
 }
 
 // All regions at one point (the sweep of tauint2, inttau2.f90:51-55,86-96,104-108):
-// signed minimum, minimum |d|, region 0's value, region L's value, the first
-// region containing the point (and its value), and the launch layer
-// (kernelsMod.f90:275-280: innermost containing region).  For the nearest-region
-// cache also: the region of the minimum |d| (k), a lower bound on every other
-// region's |d| (m2), and whether another region contains the point (negx).
+// minimum |d| and its region (k), whether some region contains the point, the
+// first one that does (nl, -1: none), and the launch layer (kernelsMod.f90:275-280:
+// innermost containing region).  For the nearest-region cache also a lower bound
+// on every other region's |d| (m2) and whether another region contains the point
+// (negx).
 template <class T>
 struct SweepOut {
-    T mn, mna, d0, dsL, dsN;
-    int nl, lay;
-    T m2;
-    int k;
-    bool negx;
+    T mna;
+    float m2;
+    int k, nl, lay;
+    bool neg, negx;
 };
 //
 // Device-memory scenes (SceneG) skip regions by their bounding spheres.  A
@@ -381,18 +380,18 @@ struct SweepOut {
 // distance -- sphere, box, capsule, segment, cylinder, torus -- under a rigid
 // transform) is skipped when the point lies farther from the sphere than the
 // smallest |d| found so far plus a rounding margin: its value is then positive
-// and larger than that minimum, so it changes none of the outputs (the signed
-// minimum only matters through its sign, and the region contains no point
-// there).  Regions 0 and L are always evaluated (their values are outputs).
+// and larger than that minimum, so it changes none of the outputs.
 //
 // only >= 0: the nearest-region cache holds, so only region `only` is evaluated
-// (mn, mna and k then describe that region alone; the caller supplies the sign
+// (mna, k and neg then describe that region alone; the caller supplies the sign
 // of the other regions).  Lanes of one warp that sweep in full and lanes that
 // sweep one region share this loop, so a warp evaluates each region at most once.
+// want_lay (the same in all lanes): the launch layer is asked for.
 template <class T, bool MODS = true, class S = SceneT<T>>
-__device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int L, int only = -1) {
-    SweepOut<T> o{(T)INFINITY, (T)INFINITY, (T)0, (T)0, (T)0, -1, 0, (T)INFINITY, 0, false};
+__device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int only, bool want_lay) {
+    SweepOut<T> o{(T)INFINITY, INFINITY, 0, -1, 0, false, false};
     T inner = (T)INFINITY;
+    float mnaf = INFINITY;
     int nneg = 0;
     bool kneg = false;
     // the warp's range of regions: all of them when a lane sweeps in full, else
@@ -404,41 +403,41 @@ __device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int L
         if (only >= 0 && i != only) continue;
         if constexpr (!std::is_same<S, SceneT<T>>::value) {
             const T br = sc.bound[4 * i + 3];
-            if (br >= (T)0 && i != 0 && i != L && o.mna < (T)INFINITY) {
+            if (br >= (T)0 && o.mna < (T)INFINITY) {
                 const T dx = p.x - sc.bound[4 * i], dy = p.y - sc.bound[4 * i + 1], dz = p.z - sc.bound[4 * i + 2];
                 const T r2 = dx * dx + dy * dy + dz * dz;
                 const T lim = o.mna + sc.cull_margin + br;
                 if (r2 > lim * lim) {
                     // outside its bounding sphere: |d| >= distance to the sphere
-                    o.m2 = fmin(o.m2, sqrt(r2) - br);
+                    o.m2 = fminf(o.m2, float_rd(sqrt(r2) - br));
                     continue;
                 }
             }
         }
         const T d = eval_region<T, MODS, S>(sc, i, p);
         const T a = fabs(d);
-        o.mn = fmin(o.mn, d);
+        const float af = float_rd(a);
+        const bool in = d < (T)0;
         if (a < o.mna) {
-            o.m2 = o.mna;
+            o.m2 = fminf(o.m2, mnaf);
+            mnaf = af;
             o.mna = a;
             o.k = i;
-            kneg = d < (T)0;
+            kneg = in;
         } else {
-            o.m2 = fmin(o.m2, a);
+            o.m2 = fminf(o.m2, af);
         }
-        nneg += d < (T)0;
-        if (i == 0) o.d0 = d;
-        if (i == L) o.dsL = d;
-        if (o.nl < 0 && d < (T)0) {
-            o.nl = i;
-            o.dsN = d;
-        }
-        const T ai = (d > (T)0) ? (T)999.0 : a;
-        if (ai < inner) {
-            inner = ai;
-            o.lay = i;
+        nneg += in;
+        if (in && o.nl < 0) o.nl = i;
+        if (want_lay) {
+            const T ai = (d > (T)0) ? (T)999.0 : a;
+            if (ai < inner) {
+                inner = ai;
+                o.lay = i;
+            }
         }
     }
+    o.neg = nneg > 0;
     o.negx = nneg - (int)kneg > 0;
     return o;
 }
@@ -965,8 +964,9 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
         // FP64 at once: the FP64 group, or a tracing step right after an FP64 sweep
         // that found the surface within half of near_band (f.near)
         bool want64 = sizeof(R) == 4 && (act == A_PRECISE || (f.near && f.mode == S_STEP));
+        const bool launching = __any_sync(__activemask(), f.mode == S_LAUNCH);
         if (!want64) {
-            sw = sweep_regions<R, MODS, S>(sc, cv<R>(pk.pos), L, only);
+            sw = sweep_regions<R, MODS, S>(sc, cv<R>(pk.pos), only, launching);
             defer = sizeof(R) == 4 && (sw.mna <= P.near_band || f.mode == S_CROSS);
             // a lane on the cache has one region to evaluate in FP64: it does so
             // now instead of waiting a round for the FP64 group (same values)
@@ -976,19 +976,17 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             }
         }
         if (want64) {
-            const SweepOut<double> s64 = sweep_regions<double, MODS, S64>(sc64, pk.pos, L, only);
-            sw = SweepOut<R>{(R)s64.mn, (R)s64.mna, (R)s64.d0, (R)s64.dsL, (R)s64.dsN, s64.nl, s64.lay,
-                             (R)s64.m2, s64.k, s64.negx};
+            const SweepOut<double> s64 = sweep_regions<double, MODS, S64>(sc64, pk.pos, only, launching);
+            sw = SweepOut<R>{(R)s64.mna, s64.m2, s64.k, s64.nl, s64.lay, s64.neg, s64.negx};
             precise = true;
         }
         if (cached) {
-            // another region containing the point keeps the signed minimum negative
-            if (f.negx && sw.mn >= (R)0) sw.mn = (R)-1;
+            sw.neg |= f.negx;  // another region contains the point
         } else {
             f.cache = kNearestCache && !ADJ && P.cache_ok && f.mode != S_CROSS;
             f.nk = sw.k;
             f.negx = sw.negx;
-            f.clear = float_rd(sw.m2);
+            f.clear = sw.m2;
         }
         f.dkup = float_ru(sw.mna);  // |d_k| here: the minimum found
         if (defer) {
@@ -996,10 +994,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             act = A_PRECISE;
         } else {
             act = A_SWEEP;
-            const R mn = sw.mn, mna = sw.mna, d0 = sw.d0, dsL = sw.dsL;
-            R dsN = sw.dsN;
-            int nl = sw.nl;
-            const int lay = sw.lay;
+            const R mna = sw.mna;
             c.sdf += N;
             f.dsdf = mna;
             const int mode = f.mode;
@@ -1008,7 +1003,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                 // top of tauint2's outer loop (:51-61).  At launch the same sweep also
                 // gives the layer (the reference evaluates the same point twice).
                 if (mode == S_LAUNCH) {
-                    pk.layer = lay;
+                    pk.layer = sw.lay;
                     c.sdf += N;
                 }
                 f.steps = 0;
@@ -1021,7 +1016,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                     act = step_or_skip<R, BATCH, ADJ, BIG>(P, pk, f, c, acc);
                 }
             } else if (mode == S_STEP) {
-                if (mn >= (R)0) {  // outside every region (:92-96)
+                if (!sw.neg) {  // outside every region (:92-96)
                     pk.tflag = true;
                     act = end_flight(P, pk);
                 } else if (++f.steps >= P.max_steps) {
@@ -1043,14 +1038,21 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                     act = sizeof(R) == 4 ? A_PRECISE : A_SWEEP + 100;
                 }
             } else {  // S_CROSS: sweep at the stepped position (:117-184)
-                if (nl < 0) {
-                    nl = 0;
-                    dsN = d0;
-                }
+                const int nl = sw.nl < 0 ? 0 : sw.nl;
                 act = A_CROSS;
                 f.mode = S_TOP;
                 if (opt_nidx<R, BATCH, BIG>(P, pk.inst, L) != opt_nidx<R, BATCH, BIG>(P, pk.inst, nl)) {
                     int which = -1;
+                    // the values of the two regions at the stepped position (the sweep's,
+                    // evaluated again: a crossing is rare, and the sweep need not carry them)
+                    R dsL, dsN;
+                    if (precise) {
+                        dsL = (R)eval_region_cold<double, MODS, S64>(sc64, L, pk.pos);
+                        dsN = (R)eval_region_cold<double, MODS, S64>(sc64, nl, pk.pos);
+                    } else {
+                        dsL = eval_region_cold<R, MODS, S>(sc, L, cv<R>(pk.pos));
+                        dsN = eval_region_cold<R, MODS, S>(sc, nl, cv<R>(pk.pos));
+                    }
                     if (dsL < (R)0 && dsN < (R)0) {
                         which = (fabs(dsL) <= fabs(dsN)) ? L : nl;
                     } else {
