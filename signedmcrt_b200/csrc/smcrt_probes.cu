@@ -239,9 +239,9 @@ __global__ void k_emit(const __grid_constant__ Params<R> P, long long first, lon
     emit(P, pk, rng);
     // the launch sweep as the transport kernel takes it: within near_band of a
     // surface, FP32 transport decides on the FP64 position with the FP64 scene
-    const SweepOut<R> o = sweep_regions<R, true>(P.sc, cv<R>(pk.pos), -1, true);
+    const SweepOut<R> o = sweep_regions<R, true, SceneT<R>, false>(P.sc, cv<R>(pk.pos), -1, -1, true);
     int lay = o.lay;
-    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true>(P.sc64, pk.pos, -1, true).lay;
+    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true, SceneT<double>, false>(P.sc64, pk.pos, -1, -1, true).lay;
     layer[i] = lay + 1;
     pos[3 * i] = pk.pos.x;
     pos[3 * i + 1] = pk.pos.y;
