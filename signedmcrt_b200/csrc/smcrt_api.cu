@@ -227,7 +227,7 @@ int check_steps(const smcrt_options* o) {
 }
 
 // The kernel's nibble table for an smcrt_group_order (0: the library's choice).
-unsigned group_order_table(int order) {
+unsigned long long group_order_table(int order) {
     return order == SMCRT_ORDER_INTERACT_LAST ? kOrderInteractLast : kOrderWalkLast;
 }
 
@@ -376,6 +376,7 @@ void fill_params(Params<R>* P, const smcrt_scene* scene, const smcrt_grid* grid,
     const bool allowed = cache_policy(scene, grid, (int)sizeof(R), &P->cache_margin);
     const int want = o ? o->nearest_cache : 0;
     P->cache_ok = allowed && want != 2 ? 1 : 0;
+    P->cache_margin_f = std::nextafter((float)P->cache_margin, INFINITY);
     P->group_order = group_order_table(o ? o->group_order : 0);
     P->normal_h = (o && o->normal_h > 0) ? o->normal_h : 1e-6;
     P->instance = o ? o->instance : 0u;
@@ -926,7 +927,7 @@ int32_t smcrt_autotune(smcrt_ctx* c, int64_t trial_packets, uint64_t seed, smcrt
     double best = -1.0;
     int best_tc = keep_tc, best_sb = keep_sb, best_cache = c->pf ? c->pf->cache_ok : c->pd->cache_ok, trials = 0;
     int best_priv = c->priv_on;
-    const unsigned keep_order = c->pf ? c->pf->group_order : c->pd->group_order;
+    const unsigned long long keep_order = c->pf ? c->pf->group_order : c->pd->group_order;
     int best_order = keep_order == kOrderInteractLast ? SMCRT_ORDER_INTERACT_LAST : SMCRT_ORDER_WALK_LAST;
     for (int tc : copies)
         for (int sb : sbins)

@@ -42,6 +42,13 @@ template <class R> __host__ __device__ __forceinline__ V3<R> operator*(V3<R> a, 
 template <class R> __host__ __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) { return {s * a.x, s * a.y, s * a.z}; }
 template <class R> __device__ __forceinline__ R dot3(V3<R> a, V3<R> b) { return (a.x * b.x) + (a.y * b.y) + (a.z * b.z); }
 template <class R> __device__ __forceinline__ R len3(V3<R> a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
+// Larger and smaller of two values; x where only c is a number's bound (a NaN x
+// gives c, as fmax does).  In FP64 a compare and two selects: fmax and fmin on
+// doubles are several instructions more.
+__device__ __forceinline__ float max_r(float x, float c) { return fmaxf(x, c); }
+__device__ __forceinline__ float min_r(float x, float c) { return fminf(x, c); }
+__device__ __forceinline__ double max_r(double x, double c) { return x > c ? x : c; }
+__device__ __forceinline__ double min_r(double x, double c) { return x < c ? x : c; }
 template <class R> __device__ __forceinline__ R clampr(R x, R lo, R hi) { return fmin(fmax(x, lo), hi); }
 template <class R> __device__ __forceinline__ R fsign(R a, R b) { return copysign(fabs(a), b); }  // Fortran sign(a,b)
 __device__ __forceinline__ void sincos_r(float x, float* s, float* c) { sincosf(x, s, c); }
@@ -75,6 +82,7 @@ enum RegionShape : int { SHAPE_GENERIC = 0, SHAPE_BOX, SHAPE_SPHERE, SHAPE_CAPSU
 template <class R>
 struct DRegion {
     int first, n, op, shape;
+    R t[3], q[7];  // a plain shape's translation and parameters
     R k, kappa, albedo, hgg, g2, nidx;
     R mus, mua;  // for the adjoint's scatter/absorption terms
 };
@@ -261,26 +269,25 @@ __device__ __forceinline__ R eval_prim(const DPrim<R>& pr, V3<R> pos) {
 
 // A region of a plain shape (RegionShape).
 template <class R>
-__device__ __forceinline__ R eval_shape(int shape, const DPrim<R>& pr, V3<R> pos) {
-    const V3<R> p{pos.x + pr.m[9], pos.y + pr.m[10], pos.z + pr.m[11]};
-    const R* q = pr.q;
-    if (shape == SHAPE_BOX) {
+__device__ __forceinline__ R eval_shape(const DRegion<R>& g, V3<R> pos) {
+    const V3<R> p{pos.x + g.t[0], pos.y + g.t[1], pos.z + g.t[2]};
+    const R* q = g.q;
+    if (g.shape == SHAPE_BOX) {
         const R dx = fabs(p.x) - q[0], dy = fabs(p.y) - q[1], dz = fabs(p.z) - q[2];
-        const R m = fmax(dx, fmax(dy, dz));
+        const R m = max_r(dx, max_r(dy, dz));
         if (m <= (R)0) return m;  // inside: the outer length is 0
-        const R mx = fmax(dx, (R)0), my = fmax(dy, (R)0), mz = fmax(dz, (R)0);
+        const R mx = max_r(dx, (R)0), my = max_r(dy, (R)0), mz = max_r(dz, (R)0);
         return sqrt(mx * mx + my * my + mz * mz);
     }
-    if (shape == SHAPE_SPHERE) return sqrt(p.x * p.x + p.y * p.y + p.z * p.z) - q[0];
+    if (g.shape == SHAPE_SPHERE) return sqrt(p.x * p.x + p.y * p.y + p.z * p.z) - q[0];
     return capsule_at(q, p, q[6]);
 }
 
-// eval_model (src/sdfs/sdf_base.f90:145-160), CSG ops src/sdfs/sdfModifiers.f90:412-475
-// S: SceneT (parameter block) or SceneG (device memory).
-template <class R, bool MODS = true, class S = SceneT<R>>
-__device__ __forceinline__ R eval_region(const S& sc, int r, V3<R> pos) {
+// eval_model (src/sdfs/sdf_base.f90:145-160), CSG ops src/sdfs/sdfModifiers.f90:412-475:
+// any region.  S: SceneT (parameter block) or SceneG (device memory).
+template <class R, bool MODS, class S>
+__device__ __forceinline__ R eval_model(const S& sc, int r, V3<R> pos) {
     const DRegion<R>& g = sc.region[r];
-    if (g.shape != SHAPE_GENERIC) return eval_shape(g.shape, sc.prim[g.first], pos);
     R d = eval_prim<R, MODS>(sc.prim[g.first], pos);
     for (int i = 1; i < g.n; ++i) {
         R d2 = eval_prim<R, MODS>(sc.prim[g.first + i], pos);
@@ -298,14 +305,26 @@ __device__ __forceinline__ R eval_region(const S& sc, int r, V3<R> pos) {
     return d;
 }
 
+
+template <class R, bool MODS = true, class S = SceneT<R>>
+__device__ __forceinline__ R eval_region(const S& sc, int r, V3<R> pos) {
+    const DRegion<R>& g = sc.region[r];
+    if (g.shape != SHAPE_GENERIC) return eval_shape(g, pos);
+    return eval_model<R, MODS, S>(sc, r, pos);
+}
+
 // calcNormal, src/sdfs/sdf_base.f90:165-189 (always double)
 template <bool MODS = true, class S = SceneT<double>>
 __device__ __forceinline__ V3<double> calc_normal(const S& sc, int r, V3<double> p, double h) {
-    const V3<double> xyy{1, -1, -1}, yyx{-1, -1, 1}, yxy{-1, 1, -1}, xxx{1, 1, 1};
-    V3<double> n = xyy * eval_region<double, MODS, S>(sc, r, p + xyy * h) +
-                   yyx * eval_region<double, MODS, S>(sc, r, p + yyx * h) +
-                   yxy * eval_region<double, MODS, S>(sc, r, p + yxy * h) +
-                   xxx * eval_region<double, MODS, S>(sc, r, p + xxx * h);
+    // the four directions (1,-1,-1), (-1,-1,1), (-1,1,-1), (1,1,1), in one loop: one
+    // copy of the region's code
+    V3<double> n{0, 0, 0};
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        const V3<double> e{i == 0 || i == 3 ? 1.0 : -1.0, i >= 2 ? 1.0 : -1.0, i & 1 ? 1.0 : -1.0};
+        const V3<double> v = e * eval_region<double, MODS, S>(sc, r, p + e * h);
+        n = i == 0 ? v : n + v;
+    }
     double t = len3(n);
     return V3<double>{n.x / t, n.y / t, n.z / t};
 }
@@ -574,8 +593,9 @@ struct Params {
     // margin of its test (FP32 transport: the FP32 sweeps' margin for both sweeps)
     int cache_ok;
     double cache_margin;
+    float cache_margin_f;  // rounded up
     // sort group of each action, one nibble per action (the round's list order)
-    unsigned group_order;
+    unsigned long long group_order;
     // shared-memory fluence privatisation (FP32 plain launches): a sub-box of
     // voxels (0-based origin, extents; priv_n cells, 0 = off) whose segments each
     // CTA sums in shared memory as 64-bit fixed point and adds to the grid once

@@ -42,6 +42,11 @@ template <class R>
 void fill_region(DRegion<R>& r, const smcrt_scene* s, const smcrt_region& g) {
     std::memset(&r, 0, sizeof(r));
     r.shape = region_shape(s, g);
+    if (r.shape != SHAPE_GENERIC) {
+        const smcrt_prim& p = s->prims[g.first_prim];
+        for (int a = 0; a < 3; ++a) r.t[a] = (R)p.transform[3][a];
+        for (int a = 0; a < 7; ++a) r.q[a] = (R)p.params[a];
+    }
     r.first = g.first_prim;
     r.n = g.nprims;
     r.op = g.op;
@@ -239,9 +244,9 @@ __global__ void k_emit(const __grid_constant__ Params<R> P, long long first, lon
     emit(P, pk, rng);
     // the launch sweep as the transport kernel takes it: within near_band of a
     // surface, FP32 transport decides on the FP64 position with the FP64 scene
-    const SweepOut<R> o = sweep_regions<R, true, SceneT<R>, false>(P.sc, cv<R>(pk.pos), -1, -1, true);
+    const SweepOut<R> o = sweep_regions<R, true, SceneT<R>, false>(P.sc, cv<R>(pk.pos), true);
     int lay = o.lay;
-    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true, SceneT<double>, false>(P.sc64, pk.pos, -1, -1, true).lay;
+    if (sizeof(R) == 4 && o.mna <= P.near_band) lay = sweep_regions<double, true, SceneT<double>, false>(P.sc64, pk.pos, true).lay;
     layer[i] = lay + 1;
     pos[3 * i] = pk.pos.x;
     pos[3 * i + 1] = pk.pos.y;

@@ -241,18 +241,18 @@ constexpr double kPrivScale = 4294967296.0;
 // One voxel segment into the fluence tally: the CTA's shared sub-box when the cell
 // lies in it, else the FP64 grid.
 template <class R, bool BATCH>
-__device__ __forceinline__ void tally_add(const Params<R>& P, int inst, int ci, int cj, int ck, int idx, R len,
+__device__ __forceinline__ void tally_add(const Params<R>& P, int inst, int ci, int cj, int ck, int idx, double len,
                                           unsigned long long* priv) {
     if (!BATCH && P.priv_n) {
         const unsigned li = (unsigned)(ci - 1 - P.priv_o[0]), lj = (unsigned)(cj - 1 - P.priv_o[1]),
                        lk = (unsigned)(ck - 1 - P.priv_o[2]);
         if (li < (unsigned)P.priv_d[0] && lj < (unsigned)P.priv_d[1] && lk < (unsigned)P.priv_d[2]) {
             atomicAdd(priv + li + P.priv_d[0] * (lj + P.priv_d[1] * lk),
-                      (unsigned long long)__double2ll_rn((double)len * kPrivScale));
+                      (unsigned long long)__double2ll_rn(len * kPrivScale));
             return;
         }
     }
-    atomicAdd(tally_grid<R, BATCH>(P, inst) + idx, (double)len);
+    atomicAdd(tally_grid<R, BATCH>(P, inst) + idx, len);
 }
 
 // The scene a kernel instantiation reads: the parameter block's, or (BIG) the
@@ -308,10 +308,32 @@ constexpr bool kNearestCache = SMCRT_NEAREST_CACHE != 0;
 #endif
 constexpr bool kCacheTop = SMCRT_CACHE_TOP != 0;
 
+// Steps of one crawl (crawl_steps): the fewest lanes of a warp that go on, and the
+// most steps, in the rounds and in drain mode.
+#ifndef SMCRT_CRAWL_MIN
+#define SMCRT_CRAWL_MIN 16
+#endif
+#ifndef SMCRT_CRAWL_MAX
+#define SMCRT_CRAWL_MAX 8
+#endif
+#ifndef SMCRT_DRAIN_CRAWL
+#define SMCRT_DRAIN_CRAWL 64
+#endif
+// A warp with at least this many lanes that need a sweep over all regions takes it
+// at once; fewer wait for the group of such sweeps.
+#ifndef SMCRT_FULL_MIN
+#define SMCRT_FULL_MIN 20
+#endif
+constexpr unsigned kFullMin = SMCRT_FULL_MIN;
+constexpr int kCrawlMin = SMCRT_CRAWL_MIN, kCrawlMax = SMCRT_CRAWL_MAX, kDrainCrawl = SMCRT_DRAIN_CRAWL;
+
 // Per-lane actions of the flattened transport loop.
 // A_PRECISE (FP32 transport): a sweep within the FP64 band of a surface, or resolving a
 // crossing, deferred to the next round and done in FP64 with the other such packets.
-enum Act : int { A_NEW = 0, A_SWEEP, A_WALK, A_CROSS, A_INTERACT, A_DEATH, A_DONE, A_PRECISE };
+// A_CRAWL: steps on the nearest-region cache inside one voxel (crawl_steps).
+// A_FULL: a sweep over all regions, beside A_SWEEP's over the kept ones.
+// A_CROSS never outlives a pass.
+enum Act : int { A_NEW = 0, A_SWEEP, A_WALK, A_CRAWL, A_INTERACT, A_DEATH, A_DONE, A_PRECISE, A_FULL, A_CROSS };
 // What the next sweep is for.
 enum SweepMode : int { S_LAUNCH = 0, S_TOP, S_STEP, S_CROSS };
 
@@ -339,6 +361,7 @@ struct Flight {
     // within half of near_band, so the next step's sweep is within near_band too
     // (a move of min|d| changes every |d| by at most that) and goes straight to FP64
     bool near;
+    R room;  // A_CRAWL: how far the packet may move inside its voxel
     // Integer voxel walk of the current step (update_grids, inttau2.f90:213-292):
     // parametric distance to the next x/y/z face, distance walked, and the cell.
     // During a crossing the same storage holds the position before the step.
@@ -355,6 +378,10 @@ struct Flight {
 };
 
 // A move of f.dsdf: off the clearance, onto the bound on |d_k|.
+template <class R>
+__device__ __forceinline__ bool cache_holds(const Params<R>& P, const Flight<R>& f) {
+    return __fadd_ru(f.dkup, P.cache_margin_f) < f.clear;
+}
 template <class R>
 __device__ __forceinline__ void cache_move(Flight<R>& f) {
     f.clear = __fsub_rd(f.clear, float_ru(f.dsdf));
@@ -403,37 +430,14 @@ __device__ __forceinline__ void key_insert(SweepOut<T>& o, unsigned key) {
 // smallest |d| found so far plus a rounding margin: its value is then positive
 // and larger than that minimum, so it changes none of the outputs.
 //
-// k1 >= 0: the nearest-region cache holds, so only the regions k1 and k2 (-1: none)
-// are evaluated (mna and nneg then describe these; the caller supplies the sign of
-// the other regions).  Lanes of one warp that sweep in full and lanes that sweep
-// their kept regions share this loop, so a warp evaluates each region at most once.
 // want_lay (the same in all lanes): the launch layer is asked for.  NL: nl is.
 template <class T, bool MODS, class S, bool NL>
-__device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int k1, int k2, bool want_lay) {
+__device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, bool want_lay) {
     SweepOut<T> o{(T)INFINITY, kKeyNone, kKeyNone, kKeyNone, 0, -1, 0};
     T inner = (T)INFINITY;
     constexpr unsigned kLow = (1u << KeyBits<S>::n) - 1u;
-    // the regions any lane of the warp needs (parameter block: at most 16, a mask;
-    // device memory: the range from the lowest to the highest)
-    constexpr bool BLOCK = std::is_same<S, SceneT<T>>::value;
-    const unsigned am = __activemask();
-    unsigned todo = 0;
-    int lo = 0, hi = 0;
-    if constexpr (BLOCK) {
-        const unsigned mine = k1 < 0 ? (1u << sc.nregions) - 1u : 1u << k1 | (k2 < 0 ? 0u : 1u << k2);
-        todo = __reduce_or_sync(am, mine);
-    } else {
-        const int a = k2 < 0 ? k1 : min(k1, k2), b = max(k1, k2);
-        lo = __reduce_min_sync(am, (unsigned)(k1 < 0 ? 0 : a));
-        hi = __reduce_max_sync(am, (unsigned)(k1 < 0 ? sc.nregions - 1 : b));
-    }
-    for (int i = lo; BLOCK ? todo != 0u : i <= hi; ++i) {
-        if constexpr (BLOCK) {
-            i = __ffs(todo) - 1;
-            todo &= todo - 1u;
-        }
-        if (k1 >= 0 && i != k1 && i != k2) continue;
-        if constexpr (!BLOCK) {
+    for (int i = 0; i < sc.nregions; ++i) {
+        if constexpr (!std::is_same<S, SceneT<T>>::value) {
             const T br = sc.bound[4 * i + 3];
             if (br >= (T)0 && o.mna < (T)INFINITY) {
                 const T dx = p.x - sc.bound[4 * i], dy = p.y - sc.bound[4 * i + 1], dz = p.z - sc.bound[4 * i + 2];
@@ -449,7 +453,7 @@ __device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int k
         const T d = eval_region<T, MODS, S>(sc, i, p);
         const T a = fabs(d);
         const bool in = d < (T)0;
-        o.mna = fmin(o.mna, a);
+        o.mna = min_r(a, o.mna);
         key_insert(o, (__float_as_uint(float_rd(a)) & ~kLow) | (unsigned)i << 1 | (unsigned)in);
         o.nneg += in;
         if (NL && in && o.nl < 0) o.nl = i;
@@ -462,6 +466,21 @@ __device__ __forceinline__ SweepOut<T> sweep_regions(const S& sc, V3<T> p, int k
         }
     }
     return o;
+}
+
+// The kept regions of the nearest-region cache at one point: minimum |d|, and
+// whether one of them contains the point.
+template <class T, bool MODS, class S>
+__device__ __forceinline__ T sweep_kept(const S& sc, V3<T> p, int k1, int k2, bool& in) {
+    T mna = (T)INFINITY;
+    in = false;
+#pragma unroll 1
+    for (int k = k1; k >= 0; k = k == k1 ? k2 : -1) {
+        const T d = eval_region<T, MODS, S>(sc, k, p);
+        mna = min_r(fabs(d), mna);
+        in = in || d < (T)0;
+    }
+    return mna;
 }
 
 // What the nearest-region cache keeps of a full sweep: the nearest region, or the
@@ -484,18 +503,6 @@ __device__ __forceinline__ void cache_keep(Flight<R>& f, const SweepOut<T>& o) {
     f.clear = two ? m3 : m2;
 }
 
-// Single-region evaluations of the crossing path.  They stay inline: an
-// out-of-line function would receive the parameter block by reference and read
-// it through generic loads instead of the constant bank.
-template <class R, bool MODS, class S>
-__device__ __forceinline__ R eval_region_cold(const S& sc, int r, V3<R> p) {
-    return eval_region<R, MODS, S>(sc, r, p);
-}
-template <bool MODS, class S>
-__device__ __forceinline__ V3<double> calc_normal_cold(const S& sc, int r, V3<double> p, double h) {
-    return calc_normal<MODS, S>(sc, r, p, h);
-}
-
 // 1-based cell of a point given in FP64 grid coordinates (position + half size),
 // update_voxels' index formula (src/inttau2.f90:433-435): FP64 transport divides
 // as the reference does; FP32 transport multiplies by the FP64 n / (2 max) (an
@@ -509,9 +516,9 @@ __device__ __forceinline__ void cell_of(const GridT<R>& g, double ox, double oy,
         cj = (int)floor((double)g.ny * oy / (2.0 * g.ymax_d)) + 1;
         ck = (int)floor((double)g.nz * oz / (2.0 * g.zmax_d)) + 1;
     } else {
-        ci = (int)floor(ox * g.sx_d) + 1;
-        cj = (int)floor(oy * g.sy_d) + 1;
-        ck = (int)floor(oz * g.sz_d) + 1;
+        ci = __double2int_rd(ox * g.sx_d) + 1;
+        cj = __double2int_rd(oy * g.sy_d) + 1;
+        ck = __double2int_rd(oz * g.sz_d) + 1;
     }
 }
 
@@ -639,6 +646,12 @@ __device__ __forceinline__ void var_flush(unsigned char* vt, double* jmean2) {
     *t.ncount = kVarEmpty;
 }
 
+// Tally index of the walk's current cell.
+template <class R>
+__device__ __forceinline__ int cell_index(const GridT<R>& g, const Flight<R>& f) {
+    return (f.w.ci - 1) + g.nx * ((f.w.cj - 1) + g.ny * (f.w.ck - 1));
+}
+
 // Voxel segments of the current step, at most SMCRT_WALK_SEGMENTS; returns true when
 // the step's walk is over.  The axis of the nearest face is picked by selects, so
 // the lanes of a warp share one face-spacing division and one code path a segment,
@@ -652,7 +665,7 @@ __device__ __forceinline__ bool walk_segments(const Params<R>& P, Pk<R>& pk, Fli
                                               unsigned char* vt, unsigned long long* priv) {
     const GridT<R>& g = P.grid;
     const V3<R>& d = pk.dir;
-    int idx = (f.w.ci - 1) + g.nx * ((f.w.cj - 1) + g.ny * (f.w.ck - 1));
+    int idx = cell_index(g, f);
 #pragma unroll 1
     for (int k = 0; k < SMCRT_WALK_SEGMENTS; ++k) {
         const R tm = fmin(f.w.tx, fmin(f.w.ty, f.w.tz));
@@ -660,7 +673,7 @@ __device__ __forceinline__ bool walk_segments(const Params<R>& P, Pk<R>& pk, Fli
         const R len = (stay ? f.dsdf : tm) - f.w.td;
         ++c.vox;
         if (ADJ) adj_track(P, pk, acc, (float)len, P.adj_w[idx]);
-        else tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, idx, len, priv);
+        else tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, idx, (double)len, priv);
         if (VAR) var_add(vt, P.jmean2, idx, (float)len, c);
         if (stay) return true;
         f.w.td = tm;
@@ -797,6 +810,124 @@ __device__ __forceinline__ int step_or_skip(const Params<R>& P, Pk<R>& pk, Fligh
     return a;
 }
 
+// The action of a packet that goes on with a tracing step: a crawl where the next
+// steps are known to be short (near a surface, or shorter than the way to the
+// nearest voxel face: at most dkup), else a sweep over the kept regions or all.
+template <class R, bool ADJ>
+__device__ __forceinline__ int next_step(const Params<R>& P, const Pk<R>& pk, Flight<R>& f) {
+    f.mode = S_STEP;
+    if (!kNearestCache || ADJ || !f.cache || !cache_holds(P, f))
+        return sizeof(R) == 4 && f.near ? A_PRECISE : A_FULL;
+    if (pk.tflag) return sizeof(R) == 4 && f.near ? A_PRECISE : A_SWEEP;
+    const R tm = fmin(f.w.tx, fmin(f.w.ty, f.w.tz));
+    f.room = f.w.td == (R)0 ? (tm - f.dsdf) - (R)1e-6 * tm : (R)-1;
+    return f.near || (R)f.dkup < f.room ? A_CRAWL : A_SWEEP;
+}
+
+// Sphere-tracing steps on the nearest-region cache inside one voxel, in registers.
+//
+// A packet closing in on a surface takes tens to thousands of ever shorter steps;
+// while the cache holds, each depends on one or two regions' values, and as long
+// as the packet stays inside its voxel it adds only its length to one cell.  Such
+// a step is a fraction of a pass of the state machine (slot traffic, sort, the
+// general sweep, cell and face distances), so these packets form a sort group of
+// their own and step here until fewer than crawl_min of the warp's lanes go on, at
+// most crawl_max times.  Every step takes the decisions of the general path on the
+// same values: a lane whose next step is anything else (the optical depth spent, a
+// voxel face ahead, a region left, the cache no longer valid) leaves before it,
+// and the general path takes that step in its next pass.
+//
+// f.room: the distance along the direction to the nearest voxel face, known from a
+// walk that ended in the cell its step began in (td == 0: the cell and the face
+// distances are those of that step's start, and later positions only move away
+// from the faces behind), less 1e-6 of the face distance for the rounding of the
+// face distances, the positions and the sum of steps.  A step shorter than that
+// stays in the cell in the general path too.  Negative: not known, found here from
+// the position as start_step finds it.
+template <class R, bool BATCH, bool MODS, bool BIG, bool VAR>
+__device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, int& act,
+                                            unsigned char* vt, unsigned long long* priv, int crawl_min,
+                                            int crawl_max) {
+    const auto& sc = scene_of<BIG>(P);
+    const auto& sc64 = scene64_of<BIG>(P);
+    using S = std::decay_t<decltype(sc)>;
+    using S64 = std::decay_t<decltype(sc64)>;
+    bool go = act == A_CRAWL, reached = false;
+    const R kap = go ? opt_kappa<R, BATCH, BIG>(P, pk.inst, pk.layer) : (R)0;
+    if (go && f.room < (R)0) {
+        const GridT<R>& g = P.grid;
+        const double ox = pk.pos.x + g.xmax_d, oy = pk.pos.y + g.ymax_d, oz = pk.pos.z + g.zmax_d;
+        cell_of<R>(g, ox, oy, oz, f.w.ci, f.w.cj, f.w.ck);
+        if (f.w.ci < 1 || f.w.ci > g.nx || f.w.cj < 1 || f.w.cj > g.ny || f.w.ck < 1 || f.w.ck > g.nz) {
+            f.room = (R)0;  // outside the grid: the general path
+        } else {
+            const R tm = fmin(first_face<R>(f.w.ci, g.vx_d, ox, pk.dir.x),
+                              fmin(first_face<R>(f.w.cj, g.vy_d, oy, pk.dir.y),
+                                   first_face<R>(f.w.ck, g.vz_d, oz, pk.dir.z)));
+            f.room = tm - (R)1e-6 * tm;
+        }
+    }
+    double sum = 0.0;
+    unsigned n = 0;
+    for (int it = 0; it < crawl_max; ++it) {
+        if (go) {
+            bool precise = sizeof(R) == 4 && f.near, in = false;
+            R mna = (R)0;
+            if (!precise) {
+                mna = sweep_kept<R, MODS, S>(sc, cv<R>(pk.pos), f.nk, f.nk2, in);
+                precise = sizeof(R) == 4 && mna <= P.near_band;
+            }
+            if (sizeof(R) == 4 && precise)
+                mna = (R)sweep_kept<double, MODS, S64>(sc64, pk.pos, f.nk, f.nk2, in);
+            const R taurun = f.taurun + mna * kap;
+            in = (in || f.negx) && f.steps + 1 < P.max_steps;
+            if (in && mna > P.eps && mna < f.room && taurun <= f.tau) {
+                ++n;
+                ++f.steps;
+                f.taurun = taurun;
+                f.dsdf = mna;
+                f.near = precise && (R)2 * mna <= P.near_band;
+                f.dkup = float_ru(mna);
+                if (VAR) var_add(vt, P.jmean2, cell_index(P.grid, f), (float)mna, c);
+                sum += (double)mna;
+                pk.pos = advance(pk.pos, mna, pk.dir);
+                cache_move(f);
+                f.room -= mna;
+                go = cache_holds(P, f);
+            } else {
+                go = false;
+                reached = in && mna <= P.eps;
+                if (reached) f.dsdf = mna;
+            }
+        }
+        if (__popc(__ballot_sync(0xffffffffu, go)) < crawl_min) break;
+    }
+    if (act != A_CRAWL) return;
+    if (n) {
+        c.sdf += n * (unsigned)sc.nregions;
+        c.steps += n;
+        c.vox += n;
+        tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, cell_index(P.grid, f), sum, priv);
+    }
+    if (reached) {
+        // the surface: as the general path takes it (inttau2.f90:99-113)
+        c.sdf += (unsigned)sc.nregions;
+        ++f.steps;
+        f.near = false;
+        if (f.taurun >= f.tau) {
+            act = end_flight(P, pk);
+        } else {
+            c.sdf += (unsigned)sc.nregions;
+            f.x.oldpos = pk.pos;
+            pk.pos = advance(pk.pos, f.dsdf + (R)2 * P.eps, pk.dir);
+            f.mode = S_CROSS;
+            act = sizeof(R) == 4 ? A_PRECISE : A_SWEEP;
+        }
+    } else if (!go) {
+        act = sizeof(R) == 4 && f.near ? A_PRECISE : cache_holds(P, f) ? A_SWEEP : A_FULL;
+    }
+}
+
 // One pass of the transport state machine for one packet: the actions in a
 // fixed order -- retire, launch, interact, sweep, cross -- then at most
 // SMCRT_WALK_SEGMENTS voxel segments.  A packet can pass through several
@@ -806,7 +937,7 @@ template <class R, int KERNEL, bool REPLAY, bool BATCH, bool ADJ, bool MODS, boo
 __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers& B, Pk<R>& pk, Flight<R>& f,
                                                Stream<R, REPLAY>& rng, Cnt& c, int& act, unsigned long long* s_cnt,
                                                double* s_mom, unsigned* s_bins, float* acc, unsigned char* vt,
-                                               unsigned long long* priv) {
+                                               unsigned long long* priv, int crawl_min, int crawl_max) {
     const auto& sc = scene_of<BIG>(P);
     const auto& sc64 = scene64_of<BIG>(P);
     using S = std::decay_t<decltype(sc)>;
@@ -922,7 +1053,12 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             act = A_SWEEP;
         }
     }
-    if (act == A_DONE) return;
+    if constexpr (kNearestCache && !ADJ) {
+        if (__any_sync(0xffffffffu, act == A_CRAWL)) {
+            crawl_steps<R, BATCH, MODS, BIG, VAR>(P, pk, f, c, act, vt, priv, crawl_min, crawl_max);
+            if (crawl_min > 1) return;
+        }
+    }
     // ---- between flights (kernelsMod.f90:285-300 / 99-134 / 408-436)
     if (act == A_INTERACT) {
         const DRegion<R>& rg = sc.region[pk.layer];
@@ -1008,37 +1144,52 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
     // signed minimum) -- the same values as the full sweep.  Boundary events
     // (crossing sweeps, launches) always sweep in full; the counters still count
     // the reference's evaluations of every region.
-    if (act == A_SWEEP || act == A_PRECISE) {
+    const bool sweeping = act == A_SWEEP || act == A_FULL || act == A_PRECISE;
+    // the cache holds for a tracing step or a flight start when the bound on
+    // |d_k| plus the margin stays below the clearance
+    const bool cached = kNearestCache && !ADJ && sweeping && f.cache &&
+                        (f.mode == S_STEP || (kCacheTop && f.mode == S_TOP)) && cache_holds(P, f);
+    const bool drain = crawl_min == 1;
+    // a few lanes that need a sweep over all regions wait for the round's group of
+    // such sweeps: the others of the warp sweep one or two regions
+    const bool full = sweeping && act != A_PRECISE && !cached;
+    const unsigned nfull = __popc(__ballot_sync(0xffffffffu, full));
+    const bool group = __any_sync(0xffffffffu, act == A_FULL);
+    const bool wait = !drain && full && nfull < kFullMin && !group;
+    if (wait) act = A_FULL;
+    if (sweeping && !wait) {
         const int L = pk.layer;
         SweepOut<R> sw{};
         bool precise = false, defer = false;
-        // the cache holds for a tracing step or a flight start when the bound on
-        // |d_k| plus the margin stays below the clearance
-        const bool cached = kNearestCache && !ADJ && f.cache && (f.mode == S_STEP || (kCacheTop && f.mode == S_TOP)) &&
-                            (double)f.dkup + P.cache_margin < (double)f.clear;
-        const int k1 = cached ? f.nk : -1, k2 = cached ? f.nk2 : -1;
         // FP64 at once: the FP64 group, or a tracing step right after an FP64 sweep
         // that found the surface within half of near_band (f.near)
         bool want64 = sizeof(R) == 4 && (act == A_PRECISE || (f.near && f.mode == S_STEP));
-        const bool launching = __any_sync(__activemask(), f.mode == S_LAUNCH);
-        if (!want64) {
-            sw = sweep_regions<R, MODS, S, sizeof(R) == 8>(sc, cv<R>(pk.pos), k1, k2, launching);
-            defer = sizeof(R) == 4 && (sw.mna <= P.near_band || f.mode == S_CROSS);
-            // a lane on the cache has one region to evaluate in FP64: it does so
-            // now instead of waiting a round for the FP64 group (same values)
-            if (defer && cached) {
-                defer = false;
-                want64 = true;
-            }
-        }
-        if (want64) {
-            const SweepOut<double> s64 = sweep_regions<double, MODS, S64, true>(sc64, pk.pos, k1, k2, launching);
-            sw = SweepOut<R>{(R)s64.mna, s64.key1, s64.key2, s64.key3, s64.nneg, s64.nl, s64.lay};
-            precise = true;
-        }
         if (cached) {
-            sw.nneg += f.negx;  // another region contains the point
+            bool in = false;
+            if (!want64) {
+                sw.mna = sweep_kept<R, MODS, S>(sc, cv<R>(pk.pos), f.nk, f.nk2, in);
+                defer = sizeof(R) == 4 && sw.mna <= P.near_band;
+                if (drain && defer) {  // now instead of in the next pass (same values)
+                    defer = false;
+                    want64 = true;
+                }
+            }
+            if (sizeof(R) == 4 && want64) {
+                sw.mna = (R)sweep_kept<double, MODS, S64>(sc64, pk.pos, f.nk, f.nk2, in);
+                precise = true;
+            }
+            sw.nneg = in || f.negx;  // another region may contain the point
         } else {
+            const bool launching = __any_sync(__activemask(), f.mode == S_LAUNCH);
+            if (!want64) {
+                sw = sweep_regions<R, MODS, S, sizeof(R) == 8>(sc, cv<R>(pk.pos), launching);
+                defer = sizeof(R) == 4 && (sw.mna <= P.near_band || f.mode == S_CROSS);
+            }
+            if (sizeof(R) == 4 && want64) {
+                const SweepOut<double> s64 = sweep_regions<double, MODS, S64, true>(sc64, pk.pos, launching);
+                sw = SweepOut<R>{(R)s64.mna, s64.key1, s64.key2, s64.key3, s64.nneg, s64.nl, s64.lay};
+                precise = true;
+            }
             f.cache = kNearestCache && !ADJ && P.cache_ok && f.mode != S_CROSS;
             cache_keep<S>(f, sw);
         }
@@ -1098,27 +1249,23 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                 if (opt_nidx<R, BATCH, BIG>(P, pk.inst, L) != opt_nidx<R, BATCH, BIG>(P, pk.inst, nl)) {
                     int which = -1;
                     // the values of the two regions at the stepped position (the sweep's,
-                    // evaluated again: a crossing is rare, and the sweep need not carry them)
-                    R dsL, dsN;
-                    if (precise) {
-                        dsL = (R)eval_region_cold<double, MODS, S64>(sc64, L, pk.pos);
-                        dsN = (R)eval_region_cold<double, MODS, S64>(sc64, nl, pk.pos);
-                    } else {
-                        dsL = eval_region_cold<R, MODS, S>(sc, L, cv<R>(pk.pos));
-                        dsN = eval_region_cold<R, MODS, S>(sc, nl, cv<R>(pk.pos));
+                    // evaluated again: a crossing is rare, and the sweep need not carry
+                    // them), then, where they decide, before the step
+                    R dsL = 0, dsN = 0, tL = 0, tN = 0;
+#pragma unroll 1
+                    for (int i = 0; i < 4; ++i) {
+                        if (i == 2 && dsL < (R)0 && dsN < (R)0) break;
+                        const int r = i & 1 ? nl : L;
+                        const V3<double> at = i < 2 ? pk.pos : f.x.oldpos;
+                        R v;
+                        // FP32 transport takes crossing sweeps in FP64
+                        if constexpr (sizeof(R) == 4) v = (R)eval_region<double, MODS, S64>(sc64, r, at);
+                        else v = eval_region<R, MODS, S>(sc, r, at);
+                        (i == 0 ? dsL : i == 1 ? dsN : i == 2 ? tL : tN) = v;
                     }
                     if (dsL < (R)0 && dsN < (R)0) {
                         which = (fabs(dsL) <= fabs(dsN)) ? L : nl;
                     } else {
-                        R tL, tN;
-                        if (precise) {
-                            tL = (R)eval_region_cold<double, MODS, S64>(sc64, L, f.x.oldpos);
-                            tN = (R)eval_region_cold<double, MODS, S64>(sc64, nl, f.x.oldpos);
-                        } else {
-                            const V3<R> of = cv<R>(f.x.oldpos);
-                            tL = eval_region_cold<R, MODS, S>(sc, L, of);
-                            tN = eval_region_cold<R, MODS, S>(sc, nl, of);
-                        }
                         if (tL < (R)0 && tN < (R)0) {
                             which = (tL >= tN) ? L : nl;
                         } else if (dsL >= (R)0 && dsN < (R)0) {
@@ -1151,7 +1298,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             const int L = pk.layer, nl = f.x.nl;
             ++c.fres;
             c.sdf += 4;
-            const V3<double> Nn = calc_normal_cold<MODS, S64>(sc64, which, pk.pos, P.normal_h);
+            const V3<double> Nn = calc_normal<MODS, S64>(sc64, which, pk.pos, P.normal_h);
             V3<double> I{(double)pk.dir.x, (double)pk.dir.y, (double)pk.dir.z};
             const double m1 = opt_nidx64<R, BATCH, BIG>(P, pk.inst, L), m2 = opt_nidx64<R, BATCH, BIG>(P, pk.inst, nl);
             const double Rf = fresnel(I, Nn, m1, m2);
@@ -1184,9 +1331,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             act = end_flight(P, pk);  // taurun >= tau ends the flight (:100)
         } else {
             f.mode = S_STEP;
-            // near a surface the next sweep is FP64: in the FP64 group, or (a
-            // lane on the cache, one region) in its own next pass
-            act = (sizeof(R) == 4 && f.near && !f.cache) ? A_PRECISE : A_SWEEP;
+            act = next_step<R, ADJ>(P, pk, f);
         }
     }
 }
@@ -1214,21 +1359,16 @@ struct SlotCount {
 // whichever warp finishes first, so the last group's chunks end each round.
 // A_DONE maps to kGroups (not listed).  Nibble `act` of an order is the group
 // of action `act`.
-constexpr unsigned kOrderWalkLast = 0x05421314u;      // sweep, interact, walk, launch
-constexpr unsigned kOrderInteractLast = 0x05431214u;  // sweep, walk, interact, launch
-constexpr int kGroups = 5;
-// Drain mode: at most this many live slots in a CTA (a few per warp), each run
-// for kDrainPasses passes per round.
+constexpr unsigned long long kOrderWalkLast = 0x207641536ull;      // ... interact, walk, launch
+constexpr unsigned long long kOrderInteractLast = 0x207651436ull;  // ... walk, interact, launch
+constexpr int kGroups = 7;
+// Drain mode: at most this many live slots in a CTA (a few per warp), run to their end.
 #ifndef SMCRT_DRAIN_LIVE_PER_WARP
 #define SMCRT_DRAIN_LIVE_PER_WARP 4
 #endif
-#ifndef SMCRT_DRAIN_PASSES
-#define SMCRT_DRAIN_PASSES 16
-#endif
 constexpr int kDrainLive = SMCRT_DRAIN_LIVE_PER_WARP * (kBlock / 32);
-constexpr int kDrainPasses = SMCRT_DRAIN_PASSES;
 static_assert(SMCRT_DRAIN_LIVE_PER_WARP <= 32, "one drain item per lane at most");
-__device__ __forceinline__ int act_group(unsigned order, int act) { return (int)((order >> (4 * act)) & 0xFu); }
+__device__ __forceinline__ int act_group(unsigned long long order, int act) { return (int)((order >> (4 * act)) & 0xFu); }
 template <class R, bool ADJ, int kSlots = SlotCount<R>::n>
 struct Slots {
     static constexpr int kRW = sizeof(R) / 4;  // 32-bit words per R
@@ -1240,8 +1380,8 @@ struct Slots {
     R dx[kSlots], dy[kSlots], dz[kSlots], w[kSlots];
     R tau[kSlots], taurun[kSlots];
     uint32_t u[kUW][kSlots];
-    // act | mode << 3 | last << 5 | tflag << 6 | adjoint pass << 7 | layer << 8 |
-    // status flags << 16 | second kept region << 24 (255: none)
+    // act | mode << 4 | last << 6 | tflag << 7 | adjoint pass << 8 | layer << 9 |
+    // status flags << 17 | second kept region << 24 (255: none)
     uint32_t meta[kSlots];
     // trace steps | nearest region << 21 | negx << 29 | cache valid << 30 | near << 31
     uint32_t steps[kSlots];
@@ -1278,13 +1418,13 @@ template <class R, bool REPLAY, bool BATCH, bool ADJ>
 __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const Params<R>& P, const Buffers& B,
                                          Pk<R>& pk, Flight<R>& f, Stream<R, REPLAY>& rng) {
     const uint32_t m = sl.meta[s];
-    const int act = (int)(m & 7u);
-    f.mode = (int)((m >> 3) & 3u);
-    f.last = (m >> 5) & 1u;
-    pk.tflag = (m >> 6) & 1u;
-    pk.phase = ADJ ? (int)((m >> 7) & 1u) : 0;
-    pk.layer = (int)((m >> 8) & 255u);
-    const int flags = (int)((m >> 16) & 255u);
+    const int act = (int)(m & 15u);
+    f.mode = (int)((m >> 4) & 3u);
+    f.last = (m >> 6) & 1u;
+    pk.tflag = (m >> 7) & 1u;
+    pk.phase = ADJ ? (int)((m >> 8) & 1u) : 0;
+    pk.layer = (int)((m >> 9) & 255u);
+    const int flags = (int)((m >> 17) & 127u);
     rng.flags = flags & STATUS_STREAM_EXHAUSTED;
     pk.flags = flags & ~STATUS_STREAM_EXHAUSTED;
     f.nk2 = (int)(m >> 24) == 255 ? -1 : (int)(m >> 24);
@@ -1334,7 +1474,12 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
         rng.ninj = (int)(o1 - o0);
     }
     constexpr int W = Slots<R, ADJ>::kRW;
-    if (act == A_WALK) {
+    if (act == A_CRAWL) {
+        f.room = get_r<R>(sl.u, 0, s);
+        f.w.ci = (int)sl.u[5 * W][s];
+        f.w.cj = (int)sl.u[5 * W + 1][s];
+        f.w.ck = (int)sl.u[5 * W + 2][s];
+    } else if (act == A_WALK) {
         f.w.tx = get_r<R>(sl.u, 0, s);
         f.w.ty = get_r<R>(sl.u, W, s);
         f.w.tz = get_r<R>(sl.u, 2 * W, s);
@@ -1343,7 +1488,7 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
         f.w.ci = (int)sl.u[5 * W][s];
         f.w.cj = (int)sl.u[5 * W + 1][s];
         f.w.ck = (int)sl.u[5 * W + 2][s];
-    } else if ((act == A_SWEEP || act == A_PRECISE) && f.mode == S_CROSS) {
+    } else if ((act == A_SWEEP || act == A_FULL || act == A_PRECISE) && f.mode == S_CROSS) {
         f.x.oldpos.x = get_r<double>(sl.u, 0, s);
         f.x.oldpos.y = get_r<double>(sl.u, 2, s);
         f.x.oldpos.z = get_r<double>(sl.u, 4, s);
@@ -1356,9 +1501,9 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
 template <class R, bool REPLAY, bool BATCH, bool ADJ>
 __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, const Pk<R>& pk, const Flight<R>& f,
                                            const Stream<R, REPLAY>& rng) {
-    sl.meta[s] = (uint32_t)act | ((uint32_t)f.mode << 3) | ((uint32_t)f.last << 5) | ((uint32_t)pk.tflag << 6) |
-                 ((uint32_t)(ADJ ? pk.phase & 1 : 0) << 7) | ((uint32_t)pk.layer << 8) |
-                 ((uint32_t)(pk.flags | rng.flags) << 16) | ((uint32_t)f.nk2 << 24);
+    sl.meta[s] = (uint32_t)act | ((uint32_t)f.mode << 4) | ((uint32_t)f.last << 6) | ((uint32_t)pk.tflag << 7) |
+                 ((uint32_t)(ADJ ? pk.phase & 1 : 0) << 8) | ((uint32_t)pk.layer << 9) |
+                 ((uint32_t)(pk.flags | rng.flags) << 17) | ((uint32_t)f.nk2 << 24);
     if (act == A_DONE) return;
     sl.px[s] = pk.pos.x;
     sl.py[s] = pk.pos.y;
@@ -1389,7 +1534,12 @@ __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, co
         sl.cpre[s] = pk.cpre;
     }
     constexpr int W = Slots<R, ADJ>::kRW;
-    if (act == A_WALK) {
+    if (act == A_CRAWL) {
+        put_r<R>(sl.u, 0, s, f.room);
+        sl.u[5 * W][s] = (uint32_t)f.w.ci;
+        sl.u[5 * W + 1][s] = (uint32_t)f.w.cj;
+        sl.u[5 * W + 2][s] = (uint32_t)f.w.ck;
+    } else if (act == A_WALK) {
         put_r<R>(sl.u, 0, s, f.w.tx);
         put_r<R>(sl.u, W, s, f.w.ty);
         put_r<R>(sl.u, 2 * W, s, f.w.tz);
@@ -1398,7 +1548,7 @@ __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, co
         sl.u[5 * W][s] = (uint32_t)f.w.ci;
         sl.u[5 * W + 1][s] = (uint32_t)f.w.cj;
         sl.u[5 * W + 2][s] = (uint32_t)f.w.ck;
-    } else if ((act == A_SWEEP || act == A_PRECISE) && f.mode == S_CROSS) {
+    } else if ((act == A_SWEEP || act == A_FULL || act == A_PRECISE) && f.mode == S_CROSS) {
         put_r<double>(sl.u, 0, s, f.x.oldpos.x);
         put_r<double>(sl.u, 2, s, f.x.oldpos.y);
         put_r<double>(sl.u, 4, s, f.x.oldpos.z);
@@ -1482,7 +1632,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
         int a[Q], rank[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            a[q] = act_group(P.group_order, (int)(sl.meta[t + q * kBlock] & 7u));
+            a[q] = act_group(P.group_order, (int)(sl.meta[t + q * kBlock] & 15u));
             rank[q] = 0;
 #pragma unroll
             for (int g = 0; g < kGroups; ++g) {
@@ -1538,34 +1688,39 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
         const int stop = s_stop;
         __syncthreads();
         if (total == 0 || stop) break;
-        // drain: few live packets left in this CTA (the end of a launch, or long
-        // histories such as a packet creeping along a wall in steps of its
-        // distance to it).  They are spread one to a few per warp (item
-        // warp + NW x lane) and each runs kDrainPasses passes before it goes back
-        // to its slot, so that a long chain of dependent steps does not wait for
-        // a sort per step.  Otherwise warps take 32-item chunks.  One call site
-        // of the pass serves both.
+        // drain: few live packets left in this CTA and none to launch (the end of a
+        // launch, or a launch of few packets).  They are spread one to a few per warp
+        // (item warp + NW x lane) and every warp runs its own to their end: long
+        // histories, such as a packet creeping along a wall in steps of its distance
+        // to it, then wait for no other warp.  Otherwise warps take 32-item chunks.
+        // One call site of the pass serves both.
         const bool drain = total <= kDrainLive;
         const int nchunks = drain ? NW : (total + 31) >> 5;
-        const int reps = drain ? kDrainPasses : 1;
         for (int chunk = warp; chunk < nchunks;) {
             const int i = drain ? chunk + NW * (int)lane : chunk * 32 + (int)lane;
-            if (i < total) {
-                const int s = s_list[i];
-                int act = load_slot<R, REPLAY, BATCH, ADJ>(sl, s, P, B, pk, f, rng);
-                for (int r = 0; r < reps; ++r) {
-                    transport_pass<R, KERNEL, REPLAY, BATCH, ADJ, MODS, BIG, VAR>(
-                        P, B, pk, f, rng, c, act, s_cnt, s_mom, s_bins, s_acc,
-                        VAR ? vbase + (size_t)s * kVarSlotBytes : nullptr, s_priv);
-                    if (act == A_DONE) break;
+            // every lane of the warp takes part in the pass (its votes are warp-wide); a
+            // lane without a packet has nothing to do
+            const int s = i < total ? (int)s_list[i] : 0;
+            int act = A_DONE;
+            if (i < total) act = load_slot<R, REPLAY, BATCH, ADJ>(sl, s, P, B, pk, f, rng);
+            for (int r = 1;; ++r) {
+                transport_pass<R, KERNEL, REPLAY, BATCH, ADJ, MODS, BIG, VAR>(
+                    P, B, pk, f, rng, c, act, s_cnt, s_mom, s_bins, s_acc,
+                    VAR ? vbase + (size_t)s * kVarSlotBytes : nullptr, s_priv, drain ? 1 : kCrawlMin,
+                    drain ? kDrainCrawl : kCrawlMax);
+                if (!drain || !__any_sync(0xffffffffu, act != A_DONE)) break;
+                if ((r & 63) == 0 && P.budget_ns && global_ns() - t0 > P.budget_ns) {
+                    atomicOr(B.status, STATUS_ABORTED);
+                    break;
                 }
-                store_slot<R, REPLAY, BATCH, ADJ>(sl, s, act, pk, f, rng);
             }
+            if (i < total) store_slot<R, REPLAY, BATCH, ADJ>(sl, s, act, pk, f, rng);
             if (drain) break;
             int next = 0;
             if (lane == 0) next = atomicAdd(&s_next, 1);
             chunk = __shfl_sync(0xffffffffu, next, 0);
         }
+        if (drain) break;
     }
     // events of packets still in flight (time budget) and since the last retire
     atomicAdd(&s_cnt[C_SDF], (unsigned long long)c.sdf);
