@@ -306,8 +306,23 @@ namespace {
 // Detector bins counted per CTA in shared memory: all of them when they fit,
 // else none.  A CTA's count of one bin is at most the packets of the launch, so
 // launches of 2^32 packets or more use the global bins.
-int shared_bins(long long nbins, long long count) {
-    return (nbins > 0 && nbins <= kMaxSharedBins && count < (1ll << 32)) ? (int)nbins : 0;
+int shared_bins(long long nbins, long long count, int room) {
+    return (nbins > 0 && nbins <= std::min(kMaxSharedBins, room) && count < (1ll << 32)) ? (int)nbins : 0;
+}
+
+// Bins that fit in shared memory beside the packet slots of a launch.
+template <class R>
+int bins_room_of(int kernel, bool replay, bool var) {
+    if (var)
+        return kernel == SMCRT_KERNEL_WEIGHT ? bins_room<SlotTraits<R, 1, false, false, false, true>>()
+                                             : bins_room<SlotTraits<R, 2, false, false, false, true>>();
+    if (replay) return bins_room<SlotTraits<R, 0, true, false, false, false>>();
+    return kernel == SMCRT_KERNEL_WEIGHT ? bins_room<SlotTraits<R, 1, false, false, false, false>>()
+           : kernel == SMCRT_KERNEL_TEST ? bins_room<SlotTraits<R, 2, false, false, false, false>>()
+                                         : bins_room<SlotTraits<R, 0, false, false, false, false>>();
+}
+int bins_room_of(int precision, int kernel, bool replay, bool var) {
+    return precision == SMCRT_FP64 ? bins_room_of<double>(kernel, replay, var) : bins_room_of<float>(kernel, replay, var);
 }
 
 // Resident CTAs per SM of the transport kernel with `smem` bytes of dynamic
@@ -333,7 +348,7 @@ int resident_per_sm(int precision, int kernel, int block, size_t smem, int block
 
 int occupancy_grid(smcrt_ctx* c, int precision, int kernel, int blocks_per_sm) {
     int per_sm = 0;
-    const size_t smem = sizeof(unsigned) * (size_t)shared_bins(c->nbins, 0);
+    const size_t smem = sizeof(unsigned) * (size_t)shared_bins(c->nbins, 0, bins_room_of(precision, kernel, false, false));
     int rc = resident_per_sm(precision, kernel, c->block, smem, blocks_per_sm, &per_sm);
     if (rc) return rc;
     c->grid_blocks = c->nsm * per_sm;
@@ -474,7 +489,8 @@ int enqueue(smcrt_ctx* c, long long first, long long count, uint64_t seed, doubl
     B.states = d_states;
     long long need = (count + c->block - 1) / c->block;
     int blocks = (int)std::min<long long>(c->grid_blocks, std::max<long long>(need, 1));
-    const int sb = c->shared_bins_on ? shared_bins(c->nbins, count) : 0;
+    const int sb = c->shared_bins_on ? shared_bins(c->nbins, count, bins_room_of(c->precision, c->kernel, replay, jm2 != nullptr))
+                                     : 0;
     int tc = 1;  // a power of two, at most one copy per CTA
     while (tc * 2 <= std::min(c->tcopies, blocks)) tc *= 2;
     int rc;
@@ -778,7 +794,8 @@ int32_t smcrt_create(const smcrt_scene* scene, const smcrt_grid* grid, const smc
                                                 std::to_string(kMaxRegions) + " regions and " +
                                                 std::to_string(kMaxPrims) + " primitives)"));
         c->variance = true;
-        const size_t slots = (size_t)(prec == SMCRT_FP64 ? SlotCount<double>::n : SlotCount<float>::n);
+        const size_t slots = (size_t)(prec == SMCRT_FP64 ? SlotTraits<double, 0, false, false, false, true>::n
+                                                         : SlotTraits<float, 0, false, false, false, true>::n);
         c->vartab_bytes = kVarSlotBytes * slots * (size_t)c->grid_blocks;
         if (cudaMalloc(&c->d_vartab, c->vartab_bytes) != cudaSuccess)
             return bail(fail(SMCRT_ERR_CUDA, "variance: cannot allocate " + std::to_string(c->vartab_bytes >> 20) +
@@ -908,7 +925,7 @@ int32_t smcrt_autotune(smcrt_ctx* c, int64_t trial_packets, uint64_t seed, smcrt
         c->copies_alloc = maxc;
     }
     std::vector<int> sbins = {1};
-    if (c->nbins > 0 && c->nbins <= kMaxSharedBins) sbins.push_back(0);
+    if (shared_bins(c->nbins, trial_packets, bins_room_of(c->precision, c->kernel, false, false)) > 0) sbins.push_back(0);
     std::vector<int> caches = {0};
     if (c->cache_allowed) caches.push_back(1);
     std::vector<int> privs = {0};
@@ -975,7 +992,8 @@ int32_t smcrt_autotune(smcrt_ctx* c, int64_t trial_packets, uint64_t seed, smcrt
         result->trials = trials;
         result->block_size = c->block;
         result->slots_per_thread =
-            c->precision == SMCRT_FP64 ? SlotCount<double>::per_thread : SlotCount<float>::per_thread;
+            c->precision == SMCRT_FP64 ? SlotTraits<double, 0, false, false, false, false>::per_thread
+                                       : SlotTraits<float, 0, false, false, false, false>::per_thread;
         result->ctas_per_sm = c->grid_blocks / std::max(1, c->nsm);
         result->nearest_cache = best_cache;
         result->shared_fluence = best_priv;
@@ -1664,7 +1682,7 @@ int run_static_t(const smcrt_scene* scene, const smcrt_grid* grid, const smcrt_s
     P.first = first;
     P.count = count;
     P.seed = seed;
-    P.sbins = shared_bins(nbins, count);
+    P.sbins = shared_bins(nbins, count, bins_room_of(sizeof(R) == 8 ? SMCRT_FP64 : SMCRT_FP32, kern, false, false));
     P.jtab[0] = jmean_dev;  // one fluence grid: no copies without allocation
     int per_sm = 0;
     cudaError_t e;

@@ -412,13 +412,15 @@ static __device__ __noinline__ uint4 philox_block(
 
 // Per-packet uniform stream: counter RNG keyed (seed, instance, packet id); in
 // replay builds (INJ) an injected uniform stream instead.  The key words live in
-// the caller's constant bank (seed, instance) and are passed at each refill.
+// the caller's constant bank (seed, instance) and are passed at each refill.  A
+// stream is its position alone: between passes no words are kept, and the block
+// that holds the position is made again at the next draw.
 template <class R, bool INJ = false>
 struct Stream {
-    uint32_t p0, p1, block;
-    uint32_t b0, b1, b2, b3;  // unconsumed Philox words, consumed from b0 (register queue)
+    uint32_t p0, p1;
+    uint32_t pos;  // Philox words consumed (INJ: uniforms consumed)
+    uint32_t b0, b1, b2, b3;  // unconsumed words of the current block, consumed from b0
     int left;
-    int ndraws;
     const double* inj;
     int ninj;
     int flags;
@@ -431,30 +433,35 @@ struct Stream {
         inst = instance;
         p0 = (uint32_t)pid;
         p1 = (uint32_t)(pid >> 32);
-        block = 0;
+        pos = 0;
         left = 0;
-        ndraws = 0;
         inj = injected;
         ninj = n;
         flags = 0;
     }
+    __device__ __forceinline__ int ndraws() const { return INJ ? (int)pos : (int)(pos / U01<R>::kWords); }
     __device__ __forceinline__ R next() {
         if (INJ) {
-            if (ndraws >= ninj) {
+            if ((int)pos >= ninj) {
                 flags |= STATUS_STREAM_EXHAUSTED;
-                ++ndraws;
+                ++pos;
                 return (R)0.5;
             }
-            return (R)inj[ndraws++];
+            return (R)inj[pos++];
         }
         if (left < U01<R>::kWords) {
-            const uint4 o = philox_block((uint32_t)seed, (uint32_t)(seed >> 32), block, inst, p0, p1);
-            b0 = o.x;
-            b1 = o.y;
+            const uint4 o = philox_block((uint32_t)seed, (uint32_t)(seed >> 32), pos >> 2, inst, p0, p1);
+            const bool two = pos & 2u, one = pos & 1u;
+            b0 = two ? o.z : o.x;
+            b1 = two ? o.w : o.y;
             b2 = o.z;
             b3 = o.w;
-            ++block;
-            left = 4;
+            if (U01<R>::kWords == 1 && one) {
+                b0 = b1;
+                b1 = b2;
+                b2 = b3;
+            }
+            left = 4 - (int)(pos & 3u);
         }
         R u;
         if (U01<R>::kWords == 1) {
@@ -468,8 +475,42 @@ struct Stream {
             b1 = b3;
         }
         left -= U01<R>::kWords;
-        ++ndraws;
+        pos += U01<R>::kWords;
         return u;
+    }
+};
+
+// Five FP32 draws of a Philox stream at once: those of one interaction (albedo,
+// bias, angle, azimuth or roulette, next optical depth).  Two blocks cover them
+// wherever the position lies, so the lanes of a warp make both together; drawing
+// one by one, each draw refills some of the lanes, and the warp pays for up to
+// five blocks.  The words are the stream's; done() moves its position past those taken.
+struct Draw5 {
+    uint32_t r[5];
+    uint32_t used;
+    __device__ __forceinline__ void fill(const Stream<float, false>& s) {
+        uint32_t a[8];
+        const uint32_t k0 = (uint32_t)s.seed, k1 = (uint32_t)(s.seed >> 32), c = s.pos >> 2;
+        philox4x32_10(k0, k1, c, s.inst, s.p0, s.p1, a);
+        philox4x32_10(k0, k1, c + 1u, s.inst, s.p0, s.p1, a + 4);
+        if (s.pos & 2u) {
+#pragma unroll
+            for (int i = 0; i < 6; ++i) a[i] = a[i + 2];
+        }
+#pragma unroll
+        for (int i = 0; i < 5; ++i) r[i] = s.pos & 1u ? a[i + 1] : a[i];
+        used = 0;
+    }
+    __device__ __forceinline__ float next() {
+        const float u = U01<float>::from(r[0], 0u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = r[i + 1];
+        ++used;
+        return u;
+    }
+    __device__ __forceinline__ void done(Stream<float, false>& s) {
+        s.pos += used;
+        s.left = 0;
     }
 };
 

@@ -29,8 +29,12 @@ static cudaError_t allow_smem(K kernel, size_t bytes) {
 cudaError_t SMCRT_CAT(launch, SMCRT_TAG, SMCRT_K)(const Params<SMCRT_R>& P, const Buffers& B, bool replay, int blocks,
                                                    int block, cudaStream_t s) {
     if (block != kBlock) return cudaErrorInvalidConfiguration;
-    const size_t smem = slots_bytes<SMCRT_R>() + priv_offset(P.sbins) + 8 * (size_t)P.priv_n;
     const bool mods = P.sc.has_mods != 0;
+    using L = SlotTraits<SMCRT_R, SMCRT_K, false, false, false, false>;
+    using LV = SlotTraits<SMCRT_R, SMCRT_K, false, false, false, true>;
+    using LR = SlotTraits<SMCRT_R, SMCRT_K, true, false, false, false>;
+    const size_t slots = P.var_tab ? slots_bytes<LV>() : replay ? slots_bytes<LR>() : slots_bytes<L>();
+    const size_t smem = slots + priv_offset(P.sbins) + 8 * (size_t)P.priv_n;
     cudaError_t e;
     if (P.var_tab) {  // second-moment run: the instantiation with the voxel-score tables
         if (replay || P.gsc.prim) return cudaErrorNotSupported;
@@ -71,7 +75,7 @@ cudaError_t SMCRT_CAT(launch_batch, SMCRT_TAG, SMCRT_K)(const Params<SMCRT_R>& P
     (void)P; (void)B; (void)blocks; (void)s;
     return cudaErrorNotSupported;
 #else
-    const size_t smem = slots_bytes<SMCRT_R>();
+    const size_t smem = slots_bytes<SlotTraits<SMCRT_R, SMCRT_K, false, true, false, false>>();
     cudaError_t e;
     if (P.sc.has_mods) {
         auto k = transport_kernel<SMCRT_R, SMCRT_K, false, true>;
@@ -95,7 +99,7 @@ cudaError_t SMCRT_CAT(launch_adjoint, SMCRT_TAG, SMCRT_K)(const Params<SMCRT_R>&
 #else
     if (sizeof(SMCRT_R) != 4) return cudaErrorNotSupported;
     if (blocks == 0) return cudaSuccess;
-    const size_t smem = slots_bytes<SMCRT_R, true>();
+    const size_t smem = slots_bytes<SlotTraits<SMCRT_R, 0, false, false, true, false>>();
     cudaError_t e;
     if (P.sc.has_mods) {
         auto k = transport_kernel<SMCRT_R, 0, false, false, true>;
@@ -120,7 +124,7 @@ cudaError_t SMCRT_CAT(priv_cells, SMCRT_TAG, SMCRT_K)(int sbins, int* cells) {
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, transport_kernel<SMCRT_R, SMCRT_K, false, false, false, false>);
     if (e != cudaSuccess) return e;
     const long long room =
-        (long long)optin - (long long)a.sharedSizeBytes - (long long)(slots_bytes<SMCRT_R>() + priv_offset(sbins));
+        (long long)optin - (long long)a.sharedSizeBytes - (long long)(slots_bytes<SlotTraits<SMCRT_R, SMCRT_K, false, false, false, false>>() + priv_offset(sbins));
     *cells = room > 0 ? (int)(room / 8) : 0;
     return cudaSuccess;
 }
@@ -128,7 +132,7 @@ cudaError_t SMCRT_CAT(priv_cells, SMCRT_TAG, SMCRT_K)(int sbins, int* cells) {
 cudaError_t SMCRT_CAT(occupancy, SMCRT_TAG, SMCRT_K)(int block, size_t sbins_bytes, int* per_sm) {
     if (block != kBlock) return cudaErrorInvalidConfiguration;
     auto k = transport_kernel<SMCRT_R, SMCRT_K, false>;
-    const size_t smem = slots_bytes<SMCRT_R>() + sbins_bytes;
+    const size_t smem = slots_bytes<SlotTraits<SMCRT_R, SMCRT_K, false, false, false, false>>() + sbins_bytes;
     cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, kBlock, smem);

@@ -20,6 +20,24 @@ namespace smcrt {
 #endif
 constexpr int kBlock = SMCRT_BLOCK;
 
+#ifndef SMCRT_SLOTS_PER_THREAD
+#define SMCRT_SLOTS_PER_THREAD 2
+#endif
+// The slots of a kernel instantiation: how many per thread (more slots give each
+// round more chunks per warp, so the wait for its slowest chunk is shorter beside
+// its work: FP32 transport takes what the 227 KiB of shared memory hold, but one less
+// in adjoint and second-moment launches, whose accumulators and tables go with it) and
+// the fields a packet needs: its weight (weight_scatter; replays report it) and its
+// own scatter count (a plain pathlength launch sums the scatters of all packets).
+template <class R_, int KERNEL, bool REPLAY, bool BATCH, bool ADJ_, bool VAR>
+struct SlotTraits {
+    using R = R_;
+    static constexpr bool ADJ = ADJ_;
+    static constexpr int per_thread = sizeof(R) == 8 ? 1 : SMCRT_SLOTS_PER_THREAD - (ADJ || VAR);
+    static constexpr int n = kBlock * per_thread;
+    static constexpr bool weight = KERNEL == SMCRT_KERNEL_WEIGHT || REPLAY;
+    static constexpr bool nscatt = KERNEL == SMCRT_KERNEL_TEST || REPLAY || BATCH || ADJ;
+};
 enum CounterIdx {
     C_PACKETS = 0,
     C_SDF,
@@ -795,6 +813,18 @@ __device__ __forceinline__ void start_flight(Flight<R>& f, Rng& rng) {
     f.taurun = 0;
 }
 
+// The draws of one interaction: made together (Draw5), or the stream itself.
+template <bool TOGETHER, class Rng>
+__device__ __forceinline__ auto draws_of(Rng& rng) -> std::conditional_t<TOGETHER, Draw5, Rng&> {
+    if constexpr (TOGETHER) {
+        Draw5 d;
+        d.fill(rng);
+        return d;
+    } else {
+        return rng;
+    }
+}
+
 // Moves through a step that starts outside the grid (no walk), then continues.
 template <class R, bool BATCH, bool ADJ, bool BIG>
 __device__ __forceinline__ int step_or_skip(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, float* acc) {
@@ -942,6 +972,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
     const auto& sc64 = scene64_of<BIG>(P);
     using S = std::decay_t<decltype(sc)>;
     using S64 = std::decay_t<decltype(sc64)>;
+    using L = SlotTraits<R, KERNEL, REPLAY, BATCH, ADJ, VAR>;
     const int N = sc.nregions;
     const R eps = P.eps;
     // ---- adjoint: the end of a packet's first pass -- add its detector term to C
@@ -966,12 +997,12 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
         // per-packet totals, summed over the retiring lanes first: one shared
         // atomic per warp (a shared-memory FP64 add is a compare-and-swap loop)
         const unsigned m = __activemask();
-        const unsigned draws = __reduce_add_sync(m, (unsigned)rng.ndraws);
-        const unsigned ns = KERNEL != SMCRT_KERNEL_WEIGHT ? __reduce_add_sync(m, (unsigned)pk.nscatt) : 0u;
+        const unsigned draws = __reduce_add_sync(m, (unsigned)rng.ndraws());
+        const unsigned ns = L::nscatt ? __reduce_add_sync(m, (unsigned)pk.nscatt) : 0u;
         if (lane_id() == (unsigned)(__ffs(m) - 1)) {
             atomicAdd(&s_cnt[C_PACKETS], (unsigned long long)__popc(m));
             atomicAdd(&s_cnt[C_DRAWS], (unsigned long long)draws);
-            if (KERNEL != SMCRT_KERNEL_WEIGHT) atomicAdd(&s_mom[24], (double)ns);
+            if (L::nscatt) atomicAdd(&s_mom[24], (double)ns);
         }
         if (pk.flags & STATUS_STEP_CAP) atomicAdd(&s_cnt[C_STEPCAP], 1ull);
         if (pk.flags & STATUS_ERROR_STATE) atomicAdd(&s_cnt[C_ERR], 1ull);
@@ -980,7 +1011,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
         if (BATCH) {
             unsigned long long* bs = P.bstats + 3ll * pk.inst;
             atomicAdd(bs + 0, 1ull);
-            atomicAdd(bs + 1, (unsigned long long)rng.ndraws);
+            atomicAdd(bs + 1, (unsigned long long)rng.ndraws());
             atomicAdd(bs + 2, (unsigned long long)pk.nscatt);
         }
         // this thread's event counts stay in registers until the kernel ends;
@@ -1002,7 +1033,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             st.weight = pk.weight;
             st.layer = pk.layer + 1;
             st.nscatt = pk.nscatt;
-            st.ndraws = rng.ndraws;
+            st.ndraws = rng.ndraws();
             st.flags = fl;
         }
         act = A_NEW;
@@ -1066,6 +1097,9 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
         const R hgg = BATCH ? P.bopt[pk.inst].hgg[pk.layer] : rg.hgg;
         const R g2 = BATCH ? P.bopt[pk.inst].g2[pk.layer] : rg.g2;
         act = A_SWEEP;
+        // FP32 counter streams: the interaction's draws together (Draw5)
+        constexpr bool kTogether = sizeof(R) == 4 && !REPLAY;
+        std::conditional_t<kTogether, Draw5, Stream<R, REPLAY>&> draw = draws_of<kTogether>(rng);
         if (KERNEL == SMCRT_KERNEL_WEIGHT) {
             const R wa = pk.weight * ((R)1 - albedo);
             pk.weight = pk.weight - wa;
@@ -1080,10 +1114,10 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                 const int cell = (ci - 1) + P.grid.nx * ((cj - 1) + P.grid.ny * (ck - 1));
                 atomicAdd(tally_grid<R, BATCH>(P, pk.inst) + cell, (double)wa);
                 if (VAR) var_add(vt, P.jmean2, cell, (float)wa, c);
-                pk.dir = hg_scatter(pk.dir, hgg, g2, rng);
+                pk.dir = hg_scatter(pk.dir, hgg, g2, draw);
                 ++c.scat;
                 if (pk.weight < (R)0.01) {  // THRESHOLD, CHANCE (constants.f90:28-30)
-                    if (rng.next() < (R)0.1) pk.weight = pk.weight / (R)0.1;
+                    if (draw.next() < (R)0.1) pk.weight = pk.weight / (R)0.1;
                     else {
                         pk.tflag = true;
                         act = A_DEATH;
@@ -1091,10 +1125,10 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                 }
             }
         } else {
-            const R ran = rng.next();
+            const R ran = draw.next();
             if (ran < albedo) {
                 R mu = 0;
-                pk.dir = hg_scatter(pk.dir, hgg, g2, rng, ADJ ? &mu : nullptr);
+                pk.dir = hg_scatter(pk.dir, hgg, g2, draw, ADJ ? &mu : nullptr);
                 if (ADJ && pk.phase) adj_scatter(P, pk, acc, mu);
                 ++c.scat;
                 pk.nscatt += 1;
@@ -1119,9 +1153,10 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             }
         }
         if (act == A_SWEEP) {
-            start_flight(f, rng);
+            start_flight(f, draw);
             f.mode = S_TOP;
         }
+        if constexpr (kTogether) draw.done(rng);
     }
     // ---- evaluate every region at the current position (the one inlined sweep)
     // Within near_band of a surface (16 FP32 ulps of the scene size, where FP32
@@ -1341,16 +1376,6 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
 // passes a packet is one slot; the union of the flight record is live only in
 // two states (a voxel walk in progress; a crossing sweep pending) and is stored
 // as raw 32-bit words.
-#ifndef SMCRT_SLOTS_PER_THREAD
-#define SMCRT_SLOTS_PER_THREAD 2
-#endif
-// Slots per thread: two for FP32 transport (124 bytes a slot); one for FP64
-// (168 bytes), so that a CTA's slots stay within the 227 KiB of shared memory.
-template <class R>
-struct SlotCount {
-    static constexpr int per_thread = sizeof(R) == 4 ? SMCRT_SLOTS_PER_THREAD : 1;
-    static constexpr int n = kBlock * per_thread;
-};
 // Sort groups of the actions a packet can wait in between rounds, in list
 // order: FP64 near-surface sweep, sweep (or a pending crossing), then walk,
 // interact and retire/launch in the order of the launch's group_order.  Each
@@ -1369,15 +1394,18 @@ constexpr int kGroups = 7;
 constexpr int kDrainLive = SMCRT_DRAIN_LIVE_PER_WARP * (kBlock / 32);
 static_assert(SMCRT_DRAIN_LIVE_PER_WARP <= 32, "one drain item per lane at most");
 __device__ __forceinline__ int act_group(unsigned long long order, int act) { return (int)((order >> (4 * act)) & 0xFu); }
-template <class R, bool ADJ, int kSlots = SlotCount<R>::n>
+template <class L>
 struct Slots {
+    using R = typename L::R;
+    static constexpr bool ADJ = L::ADJ;
+    static constexpr int kSlots = L::n;
     static constexpr int kRW = sizeof(R) / 4;  // 32-bit words per R
     // union words: walk (tx, ty, tz, td, step length, ci, cj, ck) or crossing
     // (position before the step, which, nl)
     static constexpr int kUW = 5 * kRW + 3 > 8 ? 5 * kRW + 3 : 8;
     static constexpr int kA = ADJ ? kSlots : 1;
     double px[kSlots], py[kSlots], pz[kSlots];
-    R dx[kSlots], dy[kSlots], dz[kSlots], w[kSlots];
+    R dx[kSlots], dy[kSlots], dz[kSlots], w[L::weight ? kSlots : 1];
     R tau[kSlots], taurun[kSlots];
     uint32_t u[kUW][kSlots];
     // act | mode << 4 | last << 6 | tflag << 7 | adjoint pass << 8 | layer << 9 |
@@ -1385,14 +1413,11 @@ struct Slots {
     uint32_t meta[kSlots];
     // trace steps | nearest region << 21 | negx << 29 | cache valid << 30 | near << 31
     uint32_t steps[kSlots];
-    int nscatt[kSlots];
+    int nscatt[L::nscatt ? kSlots : 1];
     // nearest-region cache: clearance and the bound on |d_k| (not in adjoint launches)
     float clr[ADJ ? 1 : kSlots], dku[ADJ ? 1 : kSlots];
-    uint32_t bl[kSlots];  // bounces (<= 1001) | rng.left << 11 | batch instance << 14
-    // Philox block counter (replay builds: the injected uniforms consumed); the
-    // draw count of a Philox stream is 4 words a block less the words left
-    uint32_t p0[kSlots], p1[kSlots], block[kSlots];
-    uint32_t b0[kSlots], b1[kSlots], b2[kSlots], b3[kSlots];
+    uint32_t bl[kSlots];  // bounces (<= 1001) | batch instance << 14
+    uint32_t p0[kSlots], p1[kSlots], rpos[kSlots];  // packet id, position in its stream
     double ctot[kA], cpre[kA];  // adjoint launches only (FP64, see Pk)
 };
 // Regions addressable by the 8-bit layer field of a slot.
@@ -1414,9 +1439,9 @@ __device__ __forceinline__ R get_r(const uint32_t (*u)[kSlots], int k, int s) {
     return (R)__longlong_as_double((long long)(((unsigned long long)u[k + 1][s] << 32) | u[k][s]));
 }
 
-template <class R, bool REPLAY, bool BATCH, bool ADJ>
-__device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const Params<R>& P, const Buffers& B,
-                                         Pk<R>& pk, Flight<R>& f, Stream<R, REPLAY>& rng) {
+template <bool REPLAY, bool BATCH, class L, class R>
+__device__ __forceinline__ int load_slot(const Slots<L>& sl, int s, const Params<R>& P, const Buffers& B, Pk<R>& pk, Flight<R>& f, Stream<R, REPLAY>& rng) {
+    constexpr bool ADJ = L::ADJ;
     const uint32_t m = sl.meta[s];
     const int act = (int)(m & 15u);
     f.mode = (int)((m >> 4) & 3u);
@@ -1432,7 +1457,7 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
     if (act == A_NEW) return act;
     pk.pos = V3<double>{sl.px[s], sl.py[s], sl.pz[s]};
     pk.dir = V3<R>{sl.dx[s], sl.dy[s], sl.dz[s]};
-    pk.weight = sl.w[s];
+    pk.weight = L::weight ? sl.w[L::weight ? s : 0] : (R)1;
     f.tau = sl.tau[s];
     f.taurun = sl.taurun[s];
     const uint32_t sw = sl.steps[s];
@@ -1443,24 +1468,14 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
     f.near = (sw >> 31) & 1u;
     f.clear = ADJ ? 0.0f : sl.clr[ADJ ? 0 : s];
     f.dkup = ADJ ? 0.0f : sl.dku[ADJ ? 0 : s];
-    pk.nscatt = sl.nscatt[s];
+    pk.nscatt = L::nscatt ? sl.nscatt[L::nscatt ? s : 0] : 0;
     const uint32_t bl = sl.bl[s];
     pk.bounces = (int)(bl & 0x7FFu);
-    rng.left = (int)((bl >> 11) & 7u);
+    rng.left = 0;
     pk.inst = BATCH ? (int)(bl >> 14) : 0;
     rng.p0 = sl.p0[s];
     rng.p1 = sl.p1[s];
-    if (REPLAY) {
-        rng.block = 0;
-        rng.ndraws = (int)sl.block[s];
-    } else {
-        rng.block = sl.block[s];
-        rng.ndraws = (int)((4u * rng.block - (unsigned)rng.left) / (unsigned)U01<R>::kWords);
-    }
-    rng.b0 = sl.b0[s];
-    rng.b1 = sl.b1[s];
-    rng.b2 = sl.b2[s];
-    rng.b3 = sl.b3[s];
+    rng.pos = sl.rpos[s];
     rng.seed = BATCH ? P.bseed[pk.inst] : P.seed;  // the stream key: the launch's, or the instance's
     if (ADJ) {
         pk.ctot = sl.ctot[s];
@@ -1473,7 +1488,7 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
         rng.inj = B.uniforms + o0;
         rng.ninj = (int)(o1 - o0);
     }
-    constexpr int W = Slots<R, ADJ>::kRW;
+    constexpr int W = Slots<L>::kRW;
     if (act == A_CRAWL) {
         f.room = get_r<R>(sl.u, 0, s);
         f.w.ci = (int)sl.u[5 * W][s];
@@ -1498,9 +1513,10 @@ __device__ __forceinline__ int load_slot(const Slots<R, ADJ>& sl, int s, const P
     return act;
 }
 
-template <class R, bool REPLAY, bool BATCH, bool ADJ>
-__device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, const Pk<R>& pk, const Flight<R>& f,
+template <bool REPLAY, bool BATCH, class L, class R>
+__device__ __forceinline__ void store_slot(Slots<L>& sl, int s, int act, const Pk<R>& pk, const Flight<R>& f,
                                            const Stream<R, REPLAY>& rng) {
+    constexpr bool ADJ = L::ADJ;
     sl.meta[s] = (uint32_t)act | ((uint32_t)f.mode << 4) | ((uint32_t)f.last << 6) | ((uint32_t)pk.tflag << 7) |
                  ((uint32_t)(ADJ ? pk.phase & 1 : 0) << 8) | ((uint32_t)pk.layer << 9) |
                  ((uint32_t)(pk.flags | rng.flags) << 17) | ((uint32_t)f.nk2 << 24);
@@ -1511,7 +1527,7 @@ __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, co
     sl.dx[s] = pk.dir.x;
     sl.dy[s] = pk.dir.y;
     sl.dz[s] = pk.dir.z;
-    sl.w[s] = pk.weight;
+    if (L::weight) sl.w[L::weight ? s : 0] = pk.weight;
     sl.tau[s] = f.tau;
     sl.taurun[s] = f.taurun;
     sl.steps[s] = (uint32_t)f.steps | ((uint32_t)f.nk << 21) | ((uint32_t)f.negx << 29) |
@@ -1520,20 +1536,16 @@ __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, co
         sl.clr[ADJ ? 0 : s] = f.clear;
         sl.dku[ADJ ? 0 : s] = f.dkup;
     }
-    sl.nscatt[s] = pk.nscatt;
-    sl.bl[s] = (uint32_t)pk.bounces | ((uint32_t)rng.left << 11) | ((uint32_t)(BATCH ? pk.inst : 0) << 14);
+    if (L::nscatt) sl.nscatt[L::nscatt ? s : 0] = pk.nscatt;
+    sl.bl[s] = (uint32_t)pk.bounces | ((uint32_t)(BATCH ? pk.inst : 0) << 14);
     sl.p0[s] = rng.p0;
     sl.p1[s] = rng.p1;
-    sl.block[s] = REPLAY ? (uint32_t)rng.ndraws : rng.block;
-    sl.b0[s] = rng.b0;
-    sl.b1[s] = rng.b1;
-    sl.b2[s] = rng.b2;
-    sl.b3[s] = rng.b3;
+    sl.rpos[s] = rng.pos;
     if (ADJ) {
         sl.ctot[s] = pk.ctot;
         sl.cpre[s] = pk.cpre;
     }
-    constexpr int W = Slots<R, ADJ>::kRW;
+    constexpr int W = Slots<L>::kRW;
     if (act == A_CRAWL) {
         put_r<R>(sl.u, 0, s, f.room);
         sl.u[5 * W][s] = (uint32_t)f.w.ci;
@@ -1561,15 +1573,20 @@ __device__ __forceinline__ void store_slot(Slots<R, ADJ>& sl, int s, int act, co
 __host__ __device__ constexpr size_t priv_offset(int sbins) { return ((size_t)sbins * 4 + 7) / 8 * 8; }
 
 // Dynamic shared memory of one CTA: the slots, then the privatized detector bins.
-template <class R, bool ADJ = false>
+template <class L>
 __host__ __device__ constexpr size_t slots_bytes() {
-    return (sizeof(Slots<R, ADJ>) + 15) / 16 * 16;
+    return (sizeof(Slots<L>) + 15) / 16 * 16;
+}
+// Detector bins that fit beside the slots (8 KiB kept for the kernel's static arrays).
+template <class L>
+__host__ __device__ constexpr int bins_room() {
+    return (int)((232448 - 8192 - (long long)slots_bytes<L>()) / 4);
 }
 
 // The persistent, compacted kernel.  KERNEL: smcrt_kernel_kind.  REPLAY:
 // injected streams.
 //
-// A CTA holds SlotCount<R>::n packets in shared memory.  Each round it counting-sorts
+// A CTA holds SlotTraits::n packets in shared memory.  Each round it counting-sorts
 // its live slots by their next action (warp ballots, stable in slot order), then
 // the warps take 32-item chunks of the sorted list, run one pass of each packet's
 // state machine and write the packets back.  A warp therefore works on 32
@@ -1586,15 +1603,16 @@ template <class R, int KERNEL, bool REPLAY, bool BATCH = false, bool ADJ = false
           bool VAR = false>
 __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(const __grid_constant__ Params<R> P,
                                                                              const Buffers B) {
-    constexpr int NS = SlotCount<R>::n;
+    using L = SlotTraits<R, KERNEL, REPLAY, BATCH, ADJ, VAR>;
+    constexpr int NS = L::n;
     __shared__ unsigned long long s_cnt[C_NUM];
     __shared__ double s_mom[25];
     __shared__ int s_stop;  // the time budget ran out
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    Slots<R, ADJ>& sl = *reinterpret_cast<Slots<R, ADJ>*>(s_dyn);
-    unsigned* s_bins = reinterpret_cast<unsigned*>(s_dyn + slots_bytes<R, ADJ>());
+    Slots<L>& sl = *reinterpret_cast<Slots<L>*>(s_dyn);
+    unsigned* s_bins = reinterpret_cast<unsigned*>(s_dyn + slots_bytes<L>());
     unsigned long long* s_priv =
-        reinterpret_cast<unsigned long long*>(s_dyn + slots_bytes<R, ADJ>() + priv_offset(P.sbins));
+        reinterpret_cast<unsigned long long*>(s_dyn + slots_bytes<L>() + priv_offset(P.sbins));
     const int t = threadIdx.x;
     const unsigned lane = lane_id();
     if (t < C_NUM) s_cnt[t] = 0ull;
@@ -1621,26 +1639,36 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     // ---- rounds: each round counting-sorts the live slots by action (warp
     // ballots and a per-warp scan, stable in slot order) and the warps take
     // 32-item chunks of the sorted list; three CTA barriers a round
-    constexpr int Q = SlotCount<R>::per_thread;
+    constexpr int Q = L::per_thread;
     constexpr int NW = kBlock / 32;
-    __shared__ int s_off[kGroups][Q][NW];
+    // slots per group, of this round and (cleared) of the next
+    __shared__ int s_group[2][8];
     __shared__ unsigned short s_list[NS];
     __shared__ int s_next;
+    if (t < 16) s_group[t >> 3][t & 7] = 0;
     const int warp = t >> 5;
-    for (;;) {
+    for (int round = 0;; round ^= 1) {
         __syncthreads();  // the previous round's slot writes are visible
-        int a[Q], rank[Q];
+        // counting sort by action: a slot's rank within its warp's slots of the group
+        // (ballots), the warp's place within the group (one shared add by the lane of
+        // that number), and the groups' places in the list
+        int a[Q], rank[Q], mine = 0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
+        for (int q = 0; q < Q; ++q)
             a[q] = act_group(P.group_order, (int)(sl.meta[t + q * kBlock] & 15u));
-            rank[q] = 0;
 #pragma unroll
-            for (int g = 0; g < kGroups; ++g) {
+        for (int g = 0; g < kGroups; ++g) {
+            int before = 0;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) {
                 const unsigned m = __ballot_sync(0xffffffffu, a[q] == g);
-                if (a[q] == g) rank[q] = __popc(m & lt);
-                if (lane == 0) s_off[g][q][warp] = __popc(m);
+                if (a[q] == g) rank[q] = before + __popc(m & lt);
+                before += __popc(m);
             }
+            if ((int)lane == g) mine = before;
         }
+        int base = 0;
+        if (mine) base = atomicAdd(&s_group[round][lane], mine);
         if (t == 0) {
             int stop = 0;
             if (P.budget_ns && global_ns() - t0 > P.budget_ns) {
@@ -1651,41 +1679,25 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             s_next = NW;
         }
         __syncthreads();
+        const int stop = s_stop;
         int total;
         {
-            constexpr int E = kGroups * Q * NW;
-            constexpr int PER = (E + 31) / 32;
-            const int* flat = &s_off[0][0][0];
-            int v[PER], sum = 0;
+            const int n = lane < 8 ? s_group[round][lane] : 0;
+            int incl = n;
 #pragma unroll
-            for (int k = 0; k < PER; ++k) {
-                const int e = (int)lane * PER + k;
-                v[k] = e < E ? flat[e] : 0;
-                sum += v[k];
-            }
-            int incl = sum;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
+            for (int d = 1; d < 8; d <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, incl, d);
                 if ((int)lane >= d) incl += y;
             }
-            total = __shfl_sync(0xffffffffu, incl, 31);
-            const int excl = incl - sum;
+            total = __shfl_sync(0xffffffffu, incl, 7);
+            const int place = incl - n + base;
 #pragma unroll
             for (int q = 0; q < Q; ++q) {
-                const int g = a[q] < kGroups ? a[q] : 0;
-                const int e = (g * Q + q) * NW + warp;
-                const int src = e / PER, k = e % PER;
-                int off = __shfl_sync(0xffffffffu, excl, src);
-#pragma unroll
-                for (int kk = 0; kk < PER; ++kk) {
-                    const int vk = __shfl_sync(0xffffffffu, v[kk], src);
-                    if (kk < k) off += vk;
-                }
+                const int off = __shfl_sync(0xffffffffu, place, a[q] & 7);
                 if (a[q] < kGroups) s_list[off + rank[q]] = (unsigned short)(t + q * kBlock);
             }
         }
-        const int stop = s_stop;
+        if (t < 8) s_group[round ^ 1][t] = 0;
         __syncthreads();
         if (total == 0 || stop) break;
         // drain: few live packets left in this CTA and none to launch (the end of a
@@ -1702,7 +1714,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             // lane without a packet has nothing to do
             const int s = i < total ? (int)s_list[i] : 0;
             int act = A_DONE;
-            if (i < total) act = load_slot<R, REPLAY, BATCH, ADJ>(sl, s, P, B, pk, f, rng);
+            if (i < total) act = load_slot<REPLAY, BATCH>(sl, s, P, B, pk, f, rng);
             for (int r = 1;; ++r) {
                 transport_pass<R, KERNEL, REPLAY, BATCH, ADJ, MODS, BIG, VAR>(
                     P, B, pk, f, rng, c, act, s_cnt, s_mom, s_bins, s_acc,
@@ -1714,7 +1726,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
                     break;
                 }
             }
-            if (i < total) store_slot<R, REPLAY, BATCH, ADJ>(sl, s, act, pk, f, rng);
+            if (i < total) store_slot<REPLAY, BATCH>(sl, s, act, pk, f, rng);
             if (drain) break;
             int next = 0;
             if (lane == 0) next = atomicAdd(&s_next, 1);
@@ -1732,7 +1744,12 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     if (VAR) atomicAdd(&s_cnt[C_VAROVF], (unsigned long long)c.varovf);
     __syncthreads();
     if (t < C_NUM && s_cnt[t]) atomicAdd(B.counters + t, s_cnt[t]);
-    if (t < 25 && s_mom[t] != 0.0) atomicAdd(B.moments + t, s_mom[t]);
+    if (t < 25) {
+        // the scatters of all packets: summed per packet, or the scatter events
+        const bool events = t == 24 && KERNEL == SMCRT_KERNEL_PATHLENGTH && !L::nscatt;
+        const double m = events ? (double)s_cnt[C_SCAT] : s_mom[t];
+        if (m != 0.0) atomicAdd(B.moments + t, m);
+    }
     for (int i = t; i < P.sbins; i += kBlock)
         if (s_bins[i]) atomicAdd(B.bins + i, (double)s_bins[i]);
     if (!ADJ && !BATCH && P.priv_n) {  // the privatised sub-box, one FP64 add per nonzero cell
