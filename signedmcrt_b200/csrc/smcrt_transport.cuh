@@ -1620,7 +1620,10 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     for (int i = t; i < P.sbins; i += kBlock) s_bins[i] = 0u;
     if (!ADJ && !BATCH)
         for (int i = t; i < P.priv_n; i += kBlock) s_priv[i] = 0ull;
-    for (int i = t; i < NS; i += kBlock) sl.meta[i] = (uint32_t)A_NEW;
+    // the CTA's share of a launch too small to fill every slot
+    const long long all = BATCH ? P.bprefix[P.ninst] : P.count;
+    const int live = (int)min((long long)NS, (all + gridDim.x - 1) / gridDim.x);
+    for (int i = t; i < NS; i += kBlock) sl.meta[i] = (uint32_t)(i < live ? A_NEW : A_DONE);
     // adjoint: per-thread gradient accumulators [3][kMaxAdjGroups][kBlock]
     __shared__ float s_acc[ADJ ? 3 * kMaxAdjGroups * kBlock : 1];
     if (ADJ)
