@@ -23,17 +23,16 @@ constexpr int kBlock = SMCRT_BLOCK;
 #ifndef SMCRT_SLOTS_PER_THREAD
 #define SMCRT_SLOTS_PER_THREAD 2
 #endif
-// The slots of a kernel instantiation: how many per thread (more slots give each
-// round more chunks per warp, so the wait for its slowest chunk is shorter beside
-// its work: FP32 transport takes what the 227 KiB of shared memory hold, but one less
-// in adjoint and second-moment launches, whose accumulators and tables go with it) and
-// the fields a packet needs: its weight (weight_scatter; replays report it) and its
-// own scatter count (a plain pathlength launch sums the scatters of all packets).
+// The slots of a kernel instantiation: two per thread in FP32 transport, one in FP64
+// (three in FP32 fit in the 227 KiB of shared memory and measured the same: 71.0
+// against 70.2 ms on 4e6 packets of sphere_water, 43.4 against 44.9 on layered_vessels),
+// and the fields a packet needs: its weight (weight_scatter; replays report it) and
+// its own scatter count (a plain pathlength launch sums the scatters of all packets).
 template <class R_, int KERNEL, bool REPLAY, bool BATCH, bool ADJ_, bool VAR>
 struct SlotTraits {
     using R = R_;
     static constexpr bool ADJ = ADJ_;
-    static constexpr int per_thread = sizeof(R) == 8 ? 1 : SMCRT_SLOTS_PER_THREAD - (ADJ || VAR);
+    static constexpr int per_thread = sizeof(R) == 8 ? 1 : SMCRT_SLOTS_PER_THREAD;
     static constexpr int n = kBlock * per_thread;
     static constexpr bool weight = KERNEL == SMCRT_KERNEL_WEIGHT || REPLAY;
     static constexpr bool nscatt = KERNEL == SMCRT_KERNEL_TEST || REPLAY || BATCH || ADJ;
@@ -746,6 +745,21 @@ __device__ __forceinline__ void adj_add(float* acc, int k, int grp, float v) {
     acc[(k * kMaxAdjGroups + grp) * kBlock + threadIdx.x] += v;
 }
 
+// Moves a warp's accumulators to the CTA's FP64 sums: an FP32 accumulator then holds
+// the terms of a few rounds, however long the launch and however many steps one
+// packet takes (15 warp sums every kAdjFlush rounds are lost in their work).
+constexpr int kAdjFlush = 8;
+__device__ __forceinline__ void adj_flush(const int ngroups, float* acc, double* grad) {
+    for (int i = 0; i < 3 * kMaxAdjGroups; ++i) {
+        if (i % kMaxAdjGroups >= ngroups) continue;
+        double v = (double)acc[i * kBlock + threadIdx.x];
+        acc[i * kBlock + threadIdx.x] = 0.0f;
+#pragma unroll
+        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (lane_id() == 0 && v != 0.0) atomicAdd(grad + i, v);
+    }
+}
+
 // Path length `len` in the packet's region, over which the fluence weight is w
 // (0 where nothing is tallied): survival term and contribution.
 template <class R>
@@ -843,10 +857,10 @@ __device__ __forceinline__ int step_or_skip(const Params<R>& P, Pk<R>& pk, Fligh
 // The action of a packet that goes on with a tracing step: a crawl where the next
 // steps are known to be short (near a surface, or shorter than the way to the
 // nearest voxel face: at most dkup), else a sweep over the kept regions or all.
-template <class R, bool ADJ>
+template <class R>
 __device__ __forceinline__ int next_step(const Params<R>& P, const Pk<R>& pk, Flight<R>& f) {
     f.mode = S_STEP;
-    if (!kNearestCache || ADJ || !f.cache || !cache_holds(P, f))
+    if (!kNearestCache || !f.cache || !cache_holds(P, f))
         return sizeof(R) == 4 && f.near ? A_PRECISE : A_FULL;
     if (pk.tflag) return sizeof(R) == 4 && f.near ? A_PRECISE : A_SWEEP;
     const R tm = fmin(f.w.tx, fmin(f.w.ty, f.w.tz));
@@ -874,8 +888,8 @@ __device__ __forceinline__ int next_step(const Params<R>& P, const Pk<R>& pk, Fl
 // face distances, the positions and the sum of steps.  A step shorter than that
 // stays in the cell in the general path too.  Negative: not known, found here from
 // the position as start_step finds it.
-template <class R, bool BATCH, bool MODS, bool BIG, bool VAR>
-__device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, int& act,
+template <class R, bool BATCH, bool ADJ, bool MODS, bool BIG, bool VAR>
+__device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, int& act, float* acc,
                                             unsigned char* vt, unsigned long long* priv, int crawl_min,
                                             int crawl_max) {
     const auto& sc = scene_of<BIG>(P);
@@ -897,6 +911,7 @@ __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Fligh
             f.room = tm - (R)1e-6 * tm;
         }
     }
+    const float w = ADJ && go && f.room > (R)0 ? P.adj_w[cell_index(P.grid, f)] : 0.0f;
     double sum = 0.0;
     unsigned n = 0;
     for (int it = 0; it < crawl_max; ++it) {
@@ -919,7 +934,8 @@ __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Fligh
                 f.near = precise && (R)2 * mna <= P.near_band;
                 f.dkup = float_ru(mna);
                 if (VAR) var_add(vt, P.jmean2, cell_index(P.grid, f), (float)mna, c);
-                sum += (double)mna;
+                if (ADJ) adj_track(P, pk, acc, (float)mna, w);
+                else sum += (double)mna;
                 pk.pos = advance(pk.pos, mna, pk.dir);
                 cache_move(f);
                 f.room -= mna;
@@ -937,7 +953,7 @@ __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Fligh
         c.sdf += n * (unsigned)sc.nregions;
         c.steps += n;
         c.vox += n;
-        tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, cell_index(P.grid, f), sum, priv);
+        if (!ADJ) tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, cell_index(P.grid, f), sum, priv);
     }
     if (reached) {
         // the surface: as the general path takes it (inttau2.f90:99-113)
@@ -1084,9 +1100,9 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             act = A_SWEEP;
         }
     }
-    if constexpr (kNearestCache && !ADJ) {
+    if constexpr (kNearestCache) {
         if (__any_sync(0xffffffffu, act == A_CRAWL)) {
-            crawl_steps<R, BATCH, MODS, BIG, VAR>(P, pk, f, c, act, vt, priv, crawl_min, crawl_max);
+            crawl_steps<R, BATCH, ADJ, MODS, BIG, VAR>(P, pk, f, c, act, acc, vt, priv, crawl_min, crawl_max);
             if (crawl_min > 1) return;
         }
     }
@@ -1182,7 +1198,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
     const bool sweeping = act == A_SWEEP || act == A_FULL || act == A_PRECISE;
     // the cache holds for a tracing step or a flight start when the bound on
     // |d_k| plus the margin stays below the clearance
-    const bool cached = kNearestCache && !ADJ && sweeping && f.cache &&
+    const bool cached = kNearestCache && sweeping && f.cache &&
                         (f.mode == S_STEP || (kCacheTop && f.mode == S_TOP)) && cache_holds(P, f);
     const bool drain = crawl_min == 1;
     // a few lanes that need a sweep over all regions wait for the round's group of
@@ -1225,7 +1241,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                 sw = SweepOut<R>{(R)s64.mna, s64.key1, s64.key2, s64.key3, s64.nneg, s64.nl, s64.lay};
                 precise = true;
             }
-            f.cache = kNearestCache && !ADJ && P.cache_ok && f.mode != S_CROSS;
+            f.cache = kNearestCache && P.cache_ok && f.mode != S_CROSS;
             cache_keep<S>(f, sw);
         }
         f.dkup = float_ru(sw.mna);  // |d_k| here: the minimum found
@@ -1366,7 +1382,7 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
             act = end_flight(P, pk);  // taurun >= tau ends the flight (:100)
         } else {
             f.mode = S_STEP;
-            act = next_step<R, ADJ>(P, pk, f);
+            act = next_step(P, pk, f);
         }
     }
 }
@@ -1414,8 +1430,8 @@ struct Slots {
     // trace steps | nearest region << 21 | negx << 29 | cache valid << 30 | near << 31
     uint32_t steps[kSlots];
     int nscatt[L::nscatt ? kSlots : 1];
-    // nearest-region cache: clearance and the bound on |d_k| (not in adjoint launches)
-    float clr[ADJ ? 1 : kSlots], dku[ADJ ? 1 : kSlots];
+    // nearest-region cache: clearance and the bound on |d_k|
+    float clr[kSlots], dku[kSlots];
     uint32_t bl[kSlots];  // bounces (<= 1001) | batch instance << 14
     uint32_t p0[kSlots], p1[kSlots], rpos[kSlots];  // packet id, position in its stream
     double ctot[kA], cpre[kA];  // adjoint launches only (FP64, see Pk)
@@ -1464,10 +1480,10 @@ __device__ __forceinline__ int load_slot(const Slots<L>& sl, int s, const Params
     f.steps = (int)(sw & 0x1FFFFFu);
     f.nk = (int)((sw >> 21) & 255u);
     f.negx = (sw >> 29) & 1u;
-    f.cache = !ADJ && ((sw >> 30) & 1u);
+    f.cache = (sw >> 30) & 1u;
     f.near = (sw >> 31) & 1u;
-    f.clear = ADJ ? 0.0f : sl.clr[ADJ ? 0 : s];
-    f.dkup = ADJ ? 0.0f : sl.dku[ADJ ? 0 : s];
+    f.clear = sl.clr[s];
+    f.dkup = sl.dku[s];
     pk.nscatt = L::nscatt ? sl.nscatt[L::nscatt ? s : 0] : 0;
     const uint32_t bl = sl.bl[s];
     pk.bounces = (int)(bl & 0x7FFu);
@@ -1531,11 +1547,9 @@ __device__ __forceinline__ void store_slot(Slots<L>& sl, int s, int act, const P
     sl.tau[s] = f.tau;
     sl.taurun[s] = f.taurun;
     sl.steps[s] = (uint32_t)f.steps | ((uint32_t)f.nk << 21) | ((uint32_t)f.negx << 29) |
-                  ((uint32_t)(!ADJ && f.cache) << 30) | ((uint32_t)f.near << 31);
-    if (!ADJ) {
-        sl.clr[ADJ ? 0 : s] = f.clear;
-        sl.dku[ADJ ? 0 : s] = f.dkup;
-    }
+                  ((uint32_t)f.cache << 30) | ((uint32_t)f.near << 31);
+    sl.clr[s] = f.clear;
+    sl.dku[s] = f.dkup;
     if (L::nscatt) sl.nscatt[L::nscatt ? s : 0] = pk.nscatt;
     sl.bl[s] = (uint32_t)pk.bounces | ((uint32_t)(BATCH ? pk.inst : 0) << 14);
     sl.p0[s] = rng.p0;
@@ -1626,8 +1640,11 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     for (int i = t; i < NS; i += kBlock) sl.meta[i] = (uint32_t)(i < live ? A_NEW : A_DONE);
     // adjoint: per-thread gradient accumulators [3][kMaxAdjGroups][kBlock]
     __shared__ float s_acc[ADJ ? 3 * kMaxAdjGroups * kBlock : 1];
-    if (ADJ)
+    __shared__ double s_grad[ADJ ? 3 * kMaxAdjGroups : 1];
+    if (ADJ) {
         for (int i = t; i < 3 * kMaxAdjGroups * kBlock; i += kBlock) s_acc[i] = 0.0f;
+        if (t < 3 * kMaxAdjGroups) s_grad[t] = 0.0;
+    }
     Pk<R> pk;
     pk.inst = 0;
     pk.phase = 0;
@@ -1650,6 +1667,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     __shared__ int s_next;
     if (t < 16) s_group[t >> 3][t & 7] = 0;
     const int warp = t >> 5;
+    int rounds = 0;
     for (int round = 0;; round ^= 1) {
         __syncthreads();  // the previous round's slot writes are visible
         // counting sort by action: a slot's rank within its warp's slots of the group
@@ -1724,6 +1742,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
                     VAR ? vbase + (size_t)s * kVarSlotBytes : nullptr, s_priv, drain ? 1 : kCrawlMin,
                     drain ? kDrainCrawl : kCrawlMax);
                 if (!drain || !__any_sync(0xffffffffu, act != A_DONE)) break;
+                if (ADJ && r % kAdjFlush == 0) adj_flush(P.adj_ngroups, s_acc, s_grad);
                 if ((r & 63) == 0 && P.budget_ns && global_ns() - t0 > P.budget_ns) {
                     atomicOr(B.status, STATUS_ABORTED);
                     break;
@@ -1736,6 +1755,7 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             chunk = __shfl_sync(0xffffffffu, next, 0);
         }
         if (drain) break;
+        if (ADJ && ++rounds % kAdjFlush == 0) adj_flush(P.adj_ngroups, s_acc, s_grad);
     }
     // events of packets still in flight (time budget) and since the last retire
     atomicAdd(&s_cnt[C_SDF], (unsigned long long)c.sdf);
@@ -1766,12 +1786,13 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             atomicAdd(grid + g, (double)(long long)v / kPrivScale);
         }
     }
-    if (ADJ && t < 3 * P.adj_ngroups) {  // thread (k, group) sums its row over the CTA's threads
-        const int k = t / P.adj_ngroups, grp = t % P.adj_ngroups;
-        const float* row = s_acc + (k * kMaxAdjGroups + grp) * kBlock;
-        double sum = 0.0;
-        for (int i = 0; i < kBlock; ++i) sum += (double)row[i];
-        atomicAdd(P.adj_out + k * P.adj_ngroups + grp, sum);
+    if (ADJ) {
+        adj_flush(P.adj_ngroups, s_acc, s_grad);
+        __syncthreads();
+        if (t < 3 * P.adj_ngroups) {
+            const int k = t / P.adj_ngroups, grp = t % P.adj_ngroups;
+            atomicAdd(P.adj_out + k * P.adj_ngroups + grp, s_grad[k * kMaxAdjGroups + grp]);
+        }
     }
 }
 
