@@ -219,8 +219,10 @@ typedef struct smcrt_options {
                               (40 KiB each, ~7.8 GB for FP32 on 148 SMs) */
     int32_t nearest_cache; /* SDF sweeps of tracing steps skip the regions a per-packet
                               nearest-region bound rules out (results unchanged):
-                              0 or 1 = on where the scene allows it (every region an
-                              exact distance under a rigid transform), 2 = off */
+                              0 or 1 = on where the scene allows it (every region a
+                              value that changes by at most the distance moved: an
+                              exact distance under a rigid transform, the same under
+                              onion and revolution, a revolved egg), 2 = off */
     int32_t shared_fluence; /* FP32 transport with a pencil source: each CTA sums the
                               fluence of a sub-box along the beam (8 x 8 cells across it,
                               as far along it as shared memory allows) in shared memory

@@ -42,6 +42,25 @@ def test_crawls_follow_the_histories_of_full_sweeps(gpu, n, kind, precision):
     assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("x", [0.0, 1.3, 2.79])
+def test_modified_regions_on_the_cache_follow_full_sweeps(gpu, x, precision):
+    """Revolved eggs and onions are on the cache (values that change by at most the
+    distance moved): the histories are those of full sweeps."""
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 41, 30, 17
+    st.grid.xmax = st.grid.ymax = st.grid.zmax = 4.0
+    st.source.position = (x, 0.2, 3.9)
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(P.setup_egg(), st, precision=precision, nearest_cache=cache, timeout_ms=20000) as tr:
+            out.append(tr.run(20000, 11))
+    on, off = out
+    for k in COUNT_KEYS:
+        assert on.stats[k] == off.stats[k], (k, on.stats[k], off.stats[k])
+    assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
+
+
 @pytest.mark.parametrize("kind", ["axis", "wall"])
 def test_crawls_match_the_oracle_in_fp64(gpu, oracle, kind):
     st, arr = stack(kind)
