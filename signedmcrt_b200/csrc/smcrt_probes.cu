@@ -24,7 +24,8 @@ void fill_prim(DPrim<R>& d, const smcrt_prim& s) {
 }
 
 // The plain shape of a region (RegionShape): a single box, sphere or capsule
-// without modifiers whose rotation part is exactly the identity.
+// without modifiers whose rotation part is exactly the identity and whose numbers
+// are finite (the plain forms' maxima do not pass over a NaN as fmax does).
 int region_shape(const smcrt_scene* s, const smcrt_region& g) {
     if (g.nprims != 1) return SHAPE_GENERIC;
     const smcrt_prim& p = s->prims[g.first_prim];
@@ -32,6 +33,10 @@ int region_shape(const smcrt_scene* s, const smcrt_region& g) {
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j)
             if (p.transform[i][j] != (i == j ? 1.0 : 0.0)) return SHAPE_GENERIC;
+    for (int i = 0; i < 3; ++i)
+        if (!std::isfinite(p.transform[3][i])) return SHAPE_GENERIC;
+    for (int i = 0; i < 7; ++i)
+        if (!std::isfinite(p.params[i])) return SHAPE_GENERIC;
     return p.kind == SMCRT_BOX       ? SHAPE_BOX
            : p.kind == SMCRT_SPHERE  ? SHAPE_SPHERE
            : p.kind == SMCRT_CAPSULE ? SHAPE_CAPSULE
@@ -219,14 +224,21 @@ __global__ void k_eval_sdf(const __grid_constant__ SceneT<R> sc, const double* p
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     V3<R> p{(R)pts[3 * i], (R)pts[3 * i + 1], (R)pts[3 * i + 2]};
-    for (int r = 0; r < sc.nregions; ++r) out[i * sc.nregions + r] = (double)eval_region(sc, r, p);
+    // at a point that is not finite the affine map's 0 x inf and 0 x NaN decide: the general path
+    const bool fin = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+    for (int r = 0; r < sc.nregions; ++r)
+        out[i * sc.nregions + r] = (double)(fin ? eval_region(sc, r, p) : eval_model<R, true>(sc, r, p));
 }
 
 __global__ void k_normal(const __grid_constant__ SceneT<double> sc, int region, double h, const double* pts,
                          long long n, double* out) {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    V3<double> nn = calc_normal(sc, region, V3<double>{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]}, h);
+    const V3<double> p{pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
+    V3<double> nn = calc_normal(sc, region, p, h);
+    // a plain shape's normal at a point that is not finite: the general path's
+    if (sc.region[region].shape != SHAPE_GENERIC && !(isfinite(p.x) && isfinite(p.y) && isfinite(p.z)))
+        nn.x = nn.y = nn.z = NAN;
     out[3 * i] = nn.x;
     out[3 * i + 1] = nn.y;
     out[3 * i + 2] = nn.z;

@@ -62,7 +62,9 @@ __device__ __forceinline__ void column_min(const SceneT<R>& sc, int r, R x, R y,
     } else {
 #pragma unroll 1
         for (int v = 0; v < kColumn; ++v) {
-            const R e = eval_region(sc, r, V3<R>{x, y, z[v]});
+            R e = eval_region(sc, r, V3<R>{x, y, z[v]});
+            // a NaN (a degenerate cone) is passed over, unless it is the first region's
+            if (first && r > 0 && e != e) e = (R)INFINITY;
 #pragma unroll
             for (int u = 0; u < kColumn; ++u)
                 if (u == v) take(u, e);

@@ -36,3 +36,15 @@ def test_render_tiles_equal_the_point_values(gpu, name, samples, precision):
     # and 0.05 of slope for twist's trigonometric terms in FP32
     tol = 64 * 4 * (2.0 ** -24 if precision == "fp32" else 2.0 ** -53) + 2.0 ** -23 * np.abs(want)
     assert np.all(np.abs(img.astype(np.float64) - want) <= tol), np.abs(img - want).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_render_passes_over_a_nan_region(gpu, precision):
+    """A degenerate cone's values are NaN everywhere; behind the first region they are
+    no minimum, wherever the first region is left out."""
+    far = S.sphere(0.1, OPT, 1, transform=S.invert(S.translate((-0.9, 0.0, 0.0))))
+    near = S.sphere(0.2, OPT, 2, transform=S.invert(S.translate((0.8, 0.0, 0.0))))
+    cone = S.cone((0.0, 0.0, 0.0), (0.0, 0.0, 0.0), 0.1, 0.1, OPT, 3)
+    samples, ext = (64, 17, 33), (1.0, 1.0, 1.0)
+    img = gpu.render(S.FlatScene([far, cone, near]), samples, ext, precision)
+    assert np.array_equal(img, gpu.render(S.FlatScene([far, near]), samples, ext, precision))

@@ -2,6 +2,8 @@
 evaluated without the affine map (RegionShape).  Its value is that of the general
 path, bit for bit: the same primitive as both children of a union is folded by the
 general path, and min(d, d) = d."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -34,3 +36,17 @@ def test_plain_shape_is_the_general_path_bit_for_bit(gpu, name, t, precision):
     pts = points(q, t)
     out = gpu.eval_sdf(S.FlatScene([prim, S.model([prim, prim], S.union)]), pts, precision)
     assert np.array_equal(out[:, 0], out[:, 1])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("name", list(SHAPES))
+def test_non_finite_points_and_parameters_take_the_general_path(gpu, name, precision):
+    nan, inf, ax = np.nan, np.inf, (-1.3, 0.0, 0.004, 1.3)
+    pts = np.array([p for a in ax for b in ax for x in (nan, inf, -inf)
+                    for p in ((x, a, b), (a, x, b), (a, b, x), (x, x, a))] + [(nan, nan, nan)])
+    prim = SHAPES[name](S.invert(S.translate((0.1, 0.0, 0.0))))
+    bad = [dataclasses.replace(prim, params=tuple(x if i == k else q for i, q in enumerate(prim.params)))
+           for k in range(len(prim.params)) for x in (nan, inf)]
+    for p, at in [(prim, pts)] + [(b, points((0.5, 0.25, 0.005), (0.1, 0.0, 0.0))) for b in bad]:
+        out = gpu.eval_sdf(S.FlatScene([p, S.model([p, p], S.union)]), at, precision)
+        assert np.array_equal(out[:, 0], out[:, 1], equal_nan=True)
