@@ -754,21 +754,6 @@ __device__ __forceinline__ void adj_add(float* acc, int k, int grp, float v) {
     acc[(k * kMaxAdjGroups + grp) * kBlock + threadIdx.x] += v;
 }
 
-// Moves a warp's accumulators to the CTA's FP64 sums: an FP32 accumulator then holds
-// the terms of a few rounds, however long the launch and however many steps one
-// packet takes (15 warp sums every kAdjFlush rounds are lost in their work).
-constexpr int kAdjFlush = 8;
-__device__ __forceinline__ void adj_flush(const int ngroups, float* acc, double* grad) {
-    for (int i = 0; i < 3 * kMaxAdjGroups; ++i) {
-        if (i % kMaxAdjGroups >= ngroups) continue;
-        double v = (double)acc[i * kBlock + threadIdx.x];
-        acc[i * kBlock + threadIdx.x] = 0.0f;
-#pragma unroll
-        for (int d = 16; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        if (lane_id() == 0 && v != 0.0) atomicAdd(grad + i, v);
-    }
-}
-
 // Path length `len` in the packet's region, over which the fluence weight is w
 // (0 where nothing is tallied): survival term and contribution.
 template <class R>
@@ -1649,11 +1634,8 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     for (int i = t; i < NS; i += kBlock) sl.meta[i] = (uint32_t)(i < live ? A_NEW : A_DONE);
     // adjoint: per-thread gradient accumulators [3][kMaxAdjGroups][kBlock]
     __shared__ float s_acc[ADJ ? 3 * kMaxAdjGroups * kBlock : 1];
-    __shared__ double s_grad[ADJ ? 3 * kMaxAdjGroups : 1];
-    if (ADJ) {
+    if (ADJ)
         for (int i = t; i < 3 * kMaxAdjGroups * kBlock; i += kBlock) s_acc[i] = 0.0f;
-        if (t < 3 * kMaxAdjGroups) s_grad[t] = 0.0;
-    }
     Pk<R> pk;
     pk.inst = 0;
     pk.phase = 0;
@@ -1676,7 +1658,6 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     __shared__ int s_next;
     if (t < 16) s_group[t >> 3][t & 7] = 0;
     const int warp = t >> 5;
-    int rounds = 0;
     for (int round = 0;; round ^= 1) {
         __syncthreads();  // the previous round's slot writes are visible
         // counting sort by action: a slot's rank within its warp's slots of the group
@@ -1751,7 +1732,6 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
                     VAR ? vbase + (size_t)s * kVarSlotBytes : nullptr, s_priv, drain ? 1 : kCrawlMin,
                     drain ? kDrainCrawl : kCrawlMax);
                 if (!drain || !__any_sync(0xffffffffu, act != A_DONE)) break;
-                if (ADJ && r % kAdjFlush == 0) adj_flush(P.adj_ngroups, s_acc, s_grad);
                 if ((r & 63) == 0 && P.budget_ns && global_ns() - t0 > P.budget_ns) {
                     atomicOr(B.status, STATUS_ABORTED);
                     break;
@@ -1764,7 +1744,6 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             chunk = __shfl_sync(0xffffffffu, next, 0);
         }
         if (drain) break;
-        if (ADJ && ++rounds % kAdjFlush == 0) adj_flush(P.adj_ngroups, s_acc, s_grad);
     }
     // events of packets still in flight (time budget) and since the last retire
     atomicAdd(&s_cnt[C_SDF], (unsigned long long)c.sdf);
@@ -1795,13 +1774,14 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
             atomicAdd(grid + g, (double)(long long)v / kPrivScale);
         }
     }
-    if (ADJ) {
-        adj_flush(P.adj_ngroups, s_acc, s_grad);
-        __syncthreads();
-        if (t < 3 * P.adj_ngroups) {
-            const int k = t / P.adj_ngroups, grp = t % P.adj_ngroups;
-            atomicAdd(P.adj_out + k * P.adj_ngroups + grp, s_grad[k * kMaxAdjGroups + grp]);
-        }
+    // thread (k, group) sums its row over the CTA's threads: one order of adding for
+    // every row, so that equal terms give equal sums
+    if (ADJ && t < 3 * P.adj_ngroups) {
+        const int k = t / P.adj_ngroups, grp = t % P.adj_ngroups;
+        const float* row = s_acc + (k * kMaxAdjGroups + grp) * kBlock;
+        double sum = 0.0;
+        for (int i = 0; i < kBlock; ++i) sum += (double)row[i];
+        atomicAdd(P.adj_out + k * P.adj_ngroups + grp, sum);
     }
 }
 
