@@ -69,3 +69,32 @@ def test_crawls_match_the_oracle_in_fp64(gpu, oracle, kind):
     o = oracle.run(arr, st, nphotons=3001, seed=7, policy=oracle.device_policy("fp64", st.grid_c()))
     diff = {k: (g.stats[k], o.stats[k]) for k in COUNT_KEYS if g.stats[k] != o.stats[k]}
     assert not diff, diff
+
+
+# (cells along the beam, distance from the wall): steps that are no multiple of an ulp of
+# the way to the voxel face (an FP32 position, a wall that is none), inside the band of
+# FP64 sweeps, up to 1.3e6 of them in a voxel of 0.1 to 0.4 cm; the last ones outside it
+WALLS = [(7, 3e-7), (5, 3e-7), (5, 3.1e-7), (20, 3e-7), (9, 1.7e-7), (20, 1.3e-6), (5, 1.02e-5), (20, 1.02e-5)]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("nz,d", WALLS)
+def test_long_crawls_end_at_the_voxel_face(gpu, nz, d, precision):
+    """A beam along a wall steps by its distance to it, all through a voxel: the lengths
+    are those of full sweeps in every voxel.  (Each packet makes 1.3 voxels' worth of
+    steps, then the step cap ends it.)"""
+    x = float(np.float32(0.9))
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 5, 3, nz
+    st.source.position = (x, 0.2, 1.0 - 1e-5)
+    arr = [S.box((2.0 * (x + d), 2.0, 2.0), S.mono(0.0, 0.0, 0.0, 1.0), 1)]
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(arr, st, precision=precision, nearest_cache=cache, timeout_ms=60000,
+                           max_trace_steps=int(1.3 * (2.0 / nz) / d)) as tr:
+            out.append(tr.run(2, 5))
+    on, off = out
+    for k in COUNT_KEYS:
+        assert on.stats[k] == off.stats[k], (k, on.stats[k], off.stats[k])
+    # the same lengths summed in another order: FP64 rounding of up to 3e6 adds
+    assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
