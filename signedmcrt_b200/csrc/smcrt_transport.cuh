@@ -654,9 +654,13 @@ __device__ __forceinline__ void var_add(unsigned char* vt, double* jmean2, int i
 // entries 32 at a time.  Each entry costs two dependent loads from device memory (the
 // tables of a launch far exceed L2), and one lane walking its packet's 80 to 240
 // entries alone held up its round for all of them (layered_vessels, 2e5 packets:
-// 32.3 -> 19.6 ms).
+// 32.3 -> 19.6 ms).  The lane that owned a table wrote it with plain stores (var_add),
+// in drain mode in the pass just before: the barrier orders these before the other
+// lanes' loads, which votes and shuffles do not.
 __device__ __forceinline__ void var_flush(unsigned char* vt, bool retires, double* jmean2) {
-    for (unsigned m = __ballot_sync(0xffffffffu, retires); m; m &= m - 1u) {
+    const unsigned all = __ballot_sync(0xffffffffu, retires);
+    if (all) __syncwarp();
+    for (unsigned m = all; m; m &= m - 1u) {
         const VarTab t = var_table((unsigned char*)__shfl_sync(0xffffffffu, (unsigned long long)vt, __ffs(m) - 1));
         const unsigned n = ~*t.ncount;
         for (unsigned k = lane_id(); k < n; k += 32) {
