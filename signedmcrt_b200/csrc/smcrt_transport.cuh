@@ -1750,8 +1750,11 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
                     VAR ? vbase + (size_t)s * kVarSlotBytes : nullptr, s_priv, drain ? 1 : kCrawlMin,
                     drain ? kDrainCrawl : kCrawlMax);
                 if (!drain || !__any_sync(0xffffffffu, act != A_DONE)) break;
-                if ((r & 63) == 0 && P.budget_ns && global_ns() - t0 > P.budget_ns) {
-                    atomicOr(B.status, STATUS_ABORTED);
+                // one decision for the warp: the lanes' clock readings may differ, and a
+                // lane that left alone would be missing from the pass's votes
+                if ((r & 63) == 0 && P.budget_ns &&
+                    __any_sync(0xffffffffu, global_ns() - t0 > P.budget_ns)) {
+                    if (lane == 0) atomicOr(B.status, STATUS_ABORTED);
                     break;
                 }
             }

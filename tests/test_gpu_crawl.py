@@ -98,3 +98,24 @@ def test_long_crawls_end_at_the_voxel_face(gpu, nz, d, precision):
         assert on.stats[k] == off.stats[k], (k, on.stats[k], off.stats[k])
     # the same lengths summed in another order: FP64 rounding of up to 3e6 adds
     assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("n", [1, 11000])
+def test_time_limit_in_launches_of_few_packets(gpu, n, precision):
+    """The time limit ends a launch whose packets (one to 75 a CTA, up to four a warp)
+    run to their end in one go, more than once, and the device goes on."""
+    from signedmcrt_b200._lib import SmcrtError
+    x, d = float(np.float32(0.9)), 1.7e-7
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 5, 3, 4
+    st.source.position = (x, 0.2, 1.0 - 1e-5)
+    arr = [S.box((2.0 * (x + d), 2.0, 2.0), S.mono(0.0, 0.0, 0.0, 1.0), 1)]
+    with gpu.Transport(arr, st, precision=precision, timeout_ms=10, max_trace_steps=2097151) as tr:
+        for _ in range(2):
+            with pytest.raises(SmcrtError, match="time limit"):
+                tr.run(n, 5)
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 5, 3, 4
+    with gpu.Transport(P.box_slab(), st, precision=precision, timeout_ms=1000) as tr:
+        assert tr.run(n, 5).stats["packets"] == n
