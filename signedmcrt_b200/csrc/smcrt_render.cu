@@ -5,15 +5,16 @@
 // Compiled without FMA contraction, so the FP64 evaluation follows the CPU
 // restatement operation for operation.
 //
-// The render is bound by the FP64 arithmetic of its distances (a 256^3 image is 67
+// The render is bound by the arithmetic of its distances (a 256^3 image is 67
 // MB, 10 us of HBM), so each CTA first finds which regions can be the minimum
 // anywhere in its tile and its voxels evaluate those alone: one or two of the eight
 // regions of layered_vessels.  Tiles of 16 x 8 x 16 voxels: small enough that few
 // regions stay, large enough that the tile's own evaluations (one a region) are few
-// beside its voxels', and 64 contiguous bytes a row.  A 256^3 FP64
-// image of layered_vessels: 491 us with every region at every voxel, 152 with the
-// tiles' regions, 100 with a thread's column sharing its x and y terms (column_min;
-// FP64: four CTAs an SM by 64 registers, 112 without).  FP32: 64 us.
+// beside its voxels', and 64 contiguous bytes a row.  A thread takes a column of
+// voxels that share their x and y terms (column_min; FP64: four CTAs an SM by 64
+// registers).  A 256^3 image of layered_vessels: FP64 500 us with every region at
+// every voxel and 126 in tiles.  Images that tiles do not suit (use_tiles) take
+// every region at every voxel.
 #include <algorithm>
 #include <cmath>
 
@@ -123,6 +124,49 @@ __global__ void __launch_bounds__(kRenderBlock, sizeof(R) == 8 ? 4 : 1) k_render
     }
 }
 
+// Every region at every voxel: one thread per voxel, consecutive threads on
+// consecutive i, so each warp writes 128 contiguous bytes of the image.
+template <class R>
+__global__ void __launch_bounds__(kRenderBlock) k_render_voxels(const __grid_constant__ SceneT<R> sc, const RenderGrid g,
+                                                                float* __restrict__ img) {
+    const long long total = g.n[0] * g.n[1] * g.n[2];
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < total; v += stride) {
+        const long long i = v % g.n[0], jk = v / g.n[0], j = jk % g.n[1], k = jk / g.n[1];
+        const V3<R> p{(R)(((double)(i + 1) - g.ns[0]) * g.w[0]), (R)(((double)(j + 1) - g.ns[1]) * g.w[1]),
+                      (R)(((double)(k + 1) - g.ns[2]) * g.w[2])};
+        // minval(ds), sdf_base.f90:332-336
+        R d = eval_region(sc, 0, p);
+        for (int r = 1; r < sc.nregions; ++r) {
+            const R e = eval_region(sc, r, p);
+            d = e < d ? e : d;
+        }
+        img[v] = (float)d;
+    }
+}
+
+// Whether an image is rendered in tiles.  In us, every voxel against tiles:
+// - enough tiles for the SMs (2.5 each): layered_vessels, FP64, 96^3 (432 tiles) 50
+//   against 47, 80^3 (250) 43 against 56;
+// - little padding: whole tiles are computed, so that a slice of 1024 x 1024 x 1 voxels
+//   (1/16 full) takes 55 against 617; 1024 x 1024 x 24 (3/4 full) 734 against 702 for
+//   layered_vessels but 225 against 259 for sphere_water;
+// - regions that tiles can leave out.  Where all can (lip), a thread's columns share
+//   their terms too.  The others (folds, modifiers) cost a column more than the same
+//   voxels alone: eggs, FP64, 256^3, 399 against 481; a scene with two such regions of
+//   seven 691 against 599 in FP64, 406 against 486 in FP32;
+// - more than one tile along each axis: the only tile spans the scene and leaves little
+//   out.  1024 x 1024 x 16: layered_vessels (8 regions) 501 against 558 and in FP32 312
+//   against 421, but sphere_water (3 regions) 155 against 131 by its columns alone.
+bool use_tiles(const smcrt_scene* scene, const RenderGrid& g, int nlip, bool fp64, long long tiles, int nsm) {
+    const int n = scene->nregions;
+    const long long total = g.n[0] * g.n[1] * g.n[2];
+    if (2 * tiles < 5LL * nsm || 5 * total < 4 * tiles * (kTx * kTy * kTz)) return false;
+    const bool thick = g.n[0] > kTx && g.n[1] > kTy && g.n[2] > kTz;
+    if (nlip == n) return thick || n <= 4;
+    return fp64 && thick && 2 * nlip > n;
+}
+
 template <class R>
 cudaError_t render_t(const smcrt_scene* scene, const RenderGrid& g, float* d_img, int nsm, cudaStream_t s) {
     SceneT<R> sc;
@@ -130,16 +174,24 @@ cudaError_t render_t(const smcrt_scene* scene, const RenderGrid& g, float* d_img
     // the regions that may be left out, and a margin far above the rounding of values
     // and coordinates (and of a transform that is rigid to 1e-9)
     unsigned lip = 0;
+    int nlip = 0;
     double scale = 1.0;
     for (int a = 0; a < 3; ++a) scale = std::fmax(scale, std::fabs(g.w[a]) * (double)(g.n[a] + 1));
     for (int r = 0; r < scene->nregions; ++r) {
         double c[3], rad;
         if (!region_bound(scene, r, c, &rad)) continue;
         lip |= 1u << r;
+        ++nlip;
         scale = std::fmax(scale, std::fabs(c[0]) + std::fabs(c[1]) + std::fabs(c[2]) + rad);
     }
     const R margin = (R)((sizeof(R) == 4 ? 1e-4 : 1e-7) * scale);
     const long long tiles = ((g.n[0] + kTx - 1) / kTx) * ((g.n[1] + kTy - 1) / kTy) * ((g.n[2] + kTz - 1) / kTz);
+    if (!use_tiles(scene, g, nlip, sizeof(R) == 8, tiles, nsm)) {
+        const long long want = (g.n[0] * g.n[1] * g.n[2] + kRenderBlock - 1) / kRenderBlock;
+        const int blocks = (int)std::min(want, 16LL * nsm);  // a few resident CTAs per SM, grid-stride beyond
+        k_render_voxels<R><<<blocks, kRenderBlock, 0, s>>>(sc, g, d_img);
+        return cudaGetLastError();
+    }
     const int blocks = (int)std::min(tiles, 8LL * nsm);  // resident CTAs, grid-stride beyond
     k_render<R><<<blocks, kRenderBlock, 0, s>>>(sc, g, lip, margin, d_img);
     return cudaGetLastError();

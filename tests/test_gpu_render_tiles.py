@@ -48,3 +48,41 @@ def test_render_passes_over_a_nan_region(gpu, precision):
     samples, ext = (64, 17, 33), (1.0, 1.0, 1.0)
     img = gpu.render(S.FlatScene([far, cone, near]), samples, ext, precision)
     assert np.array_equal(img, gpu.render(S.FlatScene([far, near]), samples, ext, precision))
+
+
+# both sides of the rule that picks tiles or single voxels: whole and partial tiles,
+# slices and rods, images with too few tiles
+SIZES = [(96, 64, 160), (95, 63, 159), (16, 200, 256), (161, 8, 300), (33, 17, 700), (1, 300, 200), (300, 1, 200),
+         (200, 300, 1), (5000, 1, 1), (64, 64, 64)]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("samples", SIZES)
+@pytest.mark.parametrize("name", ["mixed", "layered", "sphere_water"])
+def test_render_of_any_shape_equals_the_point_values(gpu, name, samples, precision):
+    test_render_tiles_equal_the_point_values(gpu, name, samples, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("samples", [(1, 1024, 1024), (1024, 1, 1024), (1024, 1024, 1)])
+def test_a_slice_costs_less_than_a_slab(gpu, samples, precision):
+    """A slice of 2^20 voxels costs well under a slab eight voxels thick: a slice computed
+    in whole tiles (15 of 16 voxels padding) costs the same as the slab."""
+    import torch
+    flat, ext = S.FlatScene(P.layered_vessels()), (1.0, 1.0, 0.605)
+
+    def us(n):
+        img = torch.empty(int(np.prod(n)), dtype=torch.float32, device="cuda")
+        s = torch.cuda.current_stream().cuda_stream
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t = []
+        for _ in range(12):
+            a.record()
+            gpu.render_device(flat, n, ext, img.data_ptr(), precision=precision, stream=s)
+            b.record()
+            torch.cuda.synchronize()
+            t.append(1e3 * a.elapsed_time(b))
+        return sorted(t[3:])[4]
+
+    slab = tuple(8 if k == 1 else k for k in samples)
+    assert us(samples) < 0.7 * us(slab)
