@@ -77,7 +77,7 @@ def _units() -> list[tuple[Path, list[str]]]:
         obj = BUILD / f"kernels_{tag}_{k}.o"
         # the FP64 variants are the accuracy mode: no FMA contraction, so their
         # arithmetic follows the CPU restatement operation for operation
-        fmad = ["--fmad=false"] if tag == "f64" else []
+        fmad = ["--fmad=false", "-DSMCRT_FMAD=0"] if tag == "f64" else []
         units.append((obj, fmad + ["-DSMCRT_R=" + rtype, "-DSMCRT_TAG=" + tag, f"-DSMCRT_K={k}",
                                    "-c", str(CSRC / "smcrt_kernels.cu"), "-o", str(obj)]))
     for name in ("smcrt_probes", "smcrt_api"):
@@ -85,7 +85,7 @@ def _units() -> list[tuple[Path, list[str]]]:
         units.append((obj, ["-c", str(CSRC / f"{name}.cu"), "-o", str(obj)]))
     # the render follows the CPU restatement operation for operation in FP64
     obj = BUILD / "smcrt_render.o"
-    units.append((obj, ["--fmad=false", "-c", str(CSRC / "smcrt_render.cu"), "-o", str(obj)]))
+    units.append((obj, ["--fmad=false", "-DSMCRT_FMAD=0", "-c", str(CSRC / "smcrt_render.cu"), "-o", str(obj)]))
     return units
 
 

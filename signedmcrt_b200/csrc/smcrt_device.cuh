@@ -117,13 +117,42 @@ struct SceneG {
     R cull_margin;
 };
 
+// The sums of products below say which product is fused with which add (mad), and
+// leave the compiler no other pair to contract.  A region's value is formed in several
+// places of a kernel (sweeps over all regions and over the kept ones, FP32 and
+// FP64, crossings), each an inlined copy of this code: a copy contracted in another way
+// would round in another way, and histories would depend on which sweep took a step.
+// SMCRT_FMAD 0 (the units built with --fmad=false): separate roundings, as the CPU
+// restatement.
+#ifndef SMCRT_FMAD
+#define SMCRT_FMAD 1
+#endif
+__device__ __forceinline__ float mad(float a, float b, float c) { return SMCRT_FMAD ? __fmaf_rn(a, b, c) : a * b + c; }
+__device__ __forceinline__ double mad(double a, double b, double c) { return SMCRT_FMAD ? __fma_rn(a, b, c) : a * b + c; }
+// a + b of products formed before, each rounded
+__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+// a b + c d + e f, and its case of squares
+template <class R>
+__device__ __forceinline__ R mad3(R a, R b, R c, R d, R e, R f) {
+    return mad(e, f, mad(a, b, c * d));
+}
+template <class R>
+__device__ __forceinline__ R dot_m(V3<R> a, V3<R> b) {
+    return mad3(a.x, b.x, a.y, b.y, a.z, b.z);
+}
+template <class R>
+__device__ __forceinline__ R len_m(V3<R> a) {
+    return sqrt(dot_m(a, a));
+}
+
 // pos .dot. transform, src/vector_class.f90:292-304
 template <class R>
 __device__ __forceinline__ V3<R> xform(const R* m, V3<R> a) {
     V3<R> d;
-    d.x = m[0] * a.x + m[3] * a.y + m[6] * a.z + m[9];
-    d.y = m[1] * a.x + m[4] * a.y + m[7] * a.z + m[10];
-    d.z = m[2] * a.x + m[5] * a.y + m[8] * a.z + m[11];
+    d.x = mad3(m[0], a.x, m[3], a.y, m[6], a.z) + m[9];
+    d.y = mad3(m[1], a.x, m[4], a.y, m[7], a.z) + m[10];
+    d.z = mad3(m[2], a.x, m[5], a.y, m[8], a.z) + m[11];
     return d;
 }
 
@@ -132,8 +161,8 @@ template <class R>
 __device__ __forceinline__ R capsule_at(const R* q, V3<R> p, R r) {
     V3<R> a{q[0], q[1], q[2]}, b{q[3], q[4], q[5]};
     V3<R> pa = p - a, ba = b - a;
-    R h = clampr(dot3(pa, ba) / dot3(ba, ba), (R)0, (R)1);
-    return len3(pa - ba * h) - r;
+    R h = clampr(dot_m(pa, ba) / dot_m(ba, ba), (R)0, (R)1);
+    return len_m(V3<R>{mad(-ba.x, h, pa.x), mad(-ba.y, h, pa.y), mad(-ba.z, h, pa.z)}) - r;
 }
 
 // Primitive SDFs, src/sdfs/sdfs.f90:494-735
@@ -144,27 +173,28 @@ __device__ __forceinline__ R eval_prim_base(const DPrim<R>& pr, V3<R> pos) {
     const R zero = 0, one = 1, half = (R)0.5;
     switch (pr.kind) {
         case SMCRT_SPHERE:
-            return sqrt(p.x * p.x + p.y * p.y + p.z * p.z) - q[0];
+            return len_m(p) - q[0];
         case SMCRT_BOX: {
             R dx = fabs(p.x) - q[0], dy = fabs(p.y) - q[1], dz = fabs(p.z) - q[2];
             R mx = fmax(dx, zero), my = fmax(dy, zero), mz = fmax(dz, zero);
-            return sqrt(mx * mx + my * my + mz * mz) + fmin(fmax(dx, fmax(dy, dz)), zero);
+            return len_m(V3<R>{mx, my, mz}) + fmin(fmax(dx, fmax(dy, dz)), zero);
         }
         case SMCRT_TORUS: {
-            R tx = sqrt(p.x * p.x + zero * zero + p.z * p.z) - q[0];
-            return sqrt(tx * tx + p.y * p.y + zero * zero) - q[1];
+            R tx = sqrt(mad(p.z, p.z, p.x * p.x)) - q[0];
+            return sqrt(mad(p.y, p.y, tx * tx)) - q[1];
         }
         case SMCRT_CYLINDER: {
             V3<R> a{q[0], q[1], q[2]}, b{q[3], q[4], q[5]};
             V3<R> ba = b - a, pa = p - a;
-            R baba = dot3(ba, ba), paba = dot3(pa, ba);
-            R x = len3(pa * baba - ba * paba) - q[6] * baba;
-            R y = fabs(paba - baba * half) - baba * half;
+            R baba = dot_m(ba, ba), paba = dot_m(pa, ba);
+            V3<R> c{mad(pa.x, baba, -(ba.x * paba)), mad(pa.y, baba, -(ba.y * paba)), mad(pa.z, baba, -(ba.z * paba))};
+            R x = mad(-q[6], baba, len_m(c));
+            R y = mad(-baba, half, fabs(mad(-baba, half, paba)));
             R x2 = x * x, y2 = (y * y) * baba, d;
             if (fmax(x, y) < zero) {
                 d = -fmin(x2, y2);
             } else {
-                if (x > zero && y > zero) d = x2 + y2;
+                if (x > zero && y > zero) d = add(x2, y2);
                 else if (x > zero) d = x2;
                 else if (y > zero) d = y2;
                 else d = zero;
@@ -172,7 +202,7 @@ __device__ __forceinline__ R eval_prim_base(const DPrim<R>& pr, V3<R> pos) {
             return fsign(sqrt(fabs(d)) / baba, d);
         }
         case SMCRT_TRIPRISM: {
-            return fmax(fabs(p.z) - q[1], fmax(fabs(p.x) * (R)0.866025 + p.y * half, -p.y) - q[0] * half);
+            return fmax(fabs(p.z) - q[1], mad(-q[0], half, fmax(mad(fabs(p.x), (R)0.866025, p.y * half), -p.y)));
         }
         case SMCRT_SEGMENT:
         case SMCRT_CAPSULE:
@@ -181,31 +211,31 @@ __device__ __forceinline__ R eval_prim_base(const DPrim<R>& pr, V3<R> pos) {
             V3<R> a{q[0], q[1], q[2]}, b{q[3], q[4], q[5]};
             R ra = q[6], rb = q[7];
             R rba = rb - ra;
-            R baba = dot3(b - a, b - a);
-            R papa = dot3(p - a, p - a);
-            R paba = dot3(p - a, b - a) / baba;
-            R x = sqrt(fmax(papa - baba * paba * paba, zero));
+            R baba = dot_m(b - a, b - a);
+            R papa = dot_m(p - a, p - a);
+            R paba = dot_m(p - a, b - a) / baba;
+            R x = sqrt(fmax(mad(-(baba * paba), paba, papa), zero));
             R cax = (paba < half) ? fmax(zero, x - ra) : fmax(zero, x - rb);
             R cay = fabs(paba - half) - half;
-            R k = rba * rba + baba;
-            R f = clampr((rba * (x - ra) + paba * baba) / k, zero, one);
-            R cbx = x - ra - f * rba;
+            R k = mad(rba, rba, baba);
+            R f = clampr(mad(rba, x - ra, paba * baba) / k, zero, one);
+            R cbx = mad(-f, rba, x - ra);
             R cby = paba - f;
             R s = (cbx < zero && cay < zero) ? -one : one;
-            return s * sqrt(fmin(cax * cax + baba * cay * cay, cbx * cbx + baba * cby * cby));
+            return s * sqrt(fmin(mad(cax, cax, baba * cay * cay), mad(cbx, cbx, baba * cby * cby)));
         }
         case SMCRT_EGG: {
             V3<R> pin{fabs(p.x), p.y, p.z};
             R r = q[0] - q[1];
             R hin = q[2] + r;
-            R l = (hin * hin - r * r) / ((R)2 * r);
-            if (pin.y <= zero) return len3(pin) - q[0];
+            R l = mad(hin, hin, -(r * r)) / ((R)2 * r);
+            if (pin.y <= zero) return len_m(pin) - q[0];
             if ((pin.y - hin) * l > pin.x * hin)
-                return len3(V3<R>{pin.x, pin.y - hin, pin.z}) - ((q[0] + l) - sqrt(hin * hin + l * l));
-            return len3(V3<R>{pin.x + l, pin.y, pin.z}) - (q[0] + l);
+                return len_m(V3<R>{pin.x, pin.y - hin, pin.z}) - ((q[0] + l) - sqrt(mad(hin, hin, l * l)));
+            return len_m(V3<R>{pin.y, pin.x + l, pin.z}) - (q[0] + l);
         }
         case SMCRT_PLANE:
-            return p.x * q[0] + p.y * q[1] + p.z * q[2];
+            return mad3(p.x, q[0], p.y, q[1], p.z, q[2]);
     }
     return zero;
 }
@@ -217,18 +247,18 @@ __device__ __forceinline__ V3<R> mod_point(int kind, const R* q, V3<R> p) {
     const R zero = 0;
     switch (kind) {
         case SMCRT_MOD_REVOLUTION:  // (|(x, z)| - o, y, 0)
-            return V3<R>{sqrt(p.x * p.x + p.z * p.z + zero * zero) - q[0], p.y, zero};
+            return V3<R>{sqrt(mad(p.x, p.x, p.z * p.z)) - q[0], p.y, zero};
         case SMCRT_MOD_ELONGATE:  // max(|p| - size, 0)
             return V3<R>{fmax(fabs(p.x) - q[0], zero), fmax(fabs(p.y) - q[1], zero), fmax(fabs(p.z) - q[2], zero)};
         case SMCRT_MOD_TWIST: {  // rotation by k z about z
             R s, c;
             sincos_r(q[0] * p.z, &s, &c);
-            return V3<R>{c * p.x - s * p.y, s * p.x + c * p.y, p.z};
+            return V3<R>{mad(c, p.x, -(s * p.y)), mad(s, p.x, c * p.y), p.z};
         }
         case SMCRT_MOD_BEND: {  // rotation by k x about z
             R s, c;
             sincos_r(q[0] * p.x, &s, &c);
-            return V3<R>{c * p.x - s * p.y, s * p.x + c * p.y, p.z};
+            return V3<R>{mad(c, p.x, -(s * p.y)), mad(s, p.x, c * p.y), p.z};
         }
         default:  // onion, extrude: the wrapped SDF sees the point itself
             return p;
@@ -243,7 +273,7 @@ __device__ __forceinline__ R mod_value(int kind, const R* q, R d, V3<R> p) {
         case SMCRT_MOD_EXTRUDE: {  // w = (d, |z| - h, 0)
             const R wy = fabs(p.z) - q[0];
             const R mx = fmax(d, zero), my = fmax(wy, zero);
-            return fmin(fmax(d, wy), zero) + sqrt(mx * mx + my * my + zero * zero);
+            return fmin(fmax(d, wy), zero) + sqrt(mad(mx, mx, my * my));
         }
         case SMCRT_MOD_ELONGATE: {
             const R qx = fabs(p.x) - q[0], qy = fabs(p.y) - q[1], qz = fabs(p.z) - q[2];
@@ -277,9 +307,9 @@ __device__ __forceinline__ R eval_shape(const DRegion<R>& g, V3<R> pos) {
         const R m = max_r(dx, max_r(dy, dz));
         if (m <= (R)0) return m;  // inside: the outer length is 0
         const R mx = max_r(dx, (R)0), my = max_r(dy, (R)0), mz = max_r(dz, (R)0);
-        return sqrt(mx * mx + my * my + mz * mz);
+        return len_m(V3<R>{mx, my, mz});
     }
-    if (g.shape == SHAPE_SPHERE) return sqrt(p.x * p.x + p.y * p.y + p.z * p.z) - q[0];
+    if (g.shape == SHAPE_SPHERE) return len_m(p) - q[0];
     return capsule_at(q, p, q[6]);
 }
 
@@ -295,7 +325,7 @@ __device__ __forceinline__ R eval_model(const S& sc, int r, V3<R> pos) {
             case SMCRT_OP_UNION: d = fmin(d, d2); break;
             case SMCRT_OP_SMOOTH_UNION: {
                 R h = fmax(g.k - fabs(d - d2), (R)0) / g.k;
-                d = fmin(d, d2) - h * h * h * g.k * ((R)1 / (R)6);
+                d = mad(-(h * h * h * g.k), (R)1 / (R)6, fmin(d, d2));
                 break;
             }
             case SMCRT_OP_SUBTRACTION: d = fmax(-d, d2); break;

@@ -556,10 +556,10 @@ template <class R, bool BATCH, bool BIG>
 __device__ __forceinline__ int start_step(const Params<R>& P, const Pk<R>& pk, Flight<R>& f, Cnt& c, bool& tflag) {
     ++c.steps;
     const R kap = opt_kappa<R, BATCH, BIG>(P, pk.inst, pk.layer);
-    const R tsdf = f.dsdf * kap;
+    const R taurun = mad(f.dsdf, kap, f.taurun);
     f.last = false;
-    if (f.taurun + tsdf <= f.tau) {
-        f.taurun = f.taurun + tsdf;
+    if (taurun <= f.tau) {
+        f.taurun = taurun;
     } else {
         f.dsdf = (f.tau - f.taurun) / kap;
         f.taurun = f.tau;
@@ -936,7 +936,7 @@ __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Fligh
             }
             if (sizeof(R) == 4 && precise)
                 mna = (R)sweep_kept<double, MODS, S64>(sc64, pk.pos, f.nk, f.nk2, in);
-            const R taurun = f.taurun + mna * kap;
+            const R taurun = mad(mna, kap, f.taurun);
             in = (in || f.negx) && f.steps + 1 < P.max_steps;
             if (in && mna > P.eps && mna < f.room && taurun <= f.tau) {
                 ++n;

@@ -119,3 +119,110 @@ def test_time_limit_in_launches_of_few_packets(gpu, n, precision):
     st.grid.nxg, st.grid.nyg, st.grid.nzg = 5, 3, 4
     with gpu.Transport(P.box_slab(), st, precision=precision, timeout_ms=1000) as tr:
         assert tr.run(n, 5).stats["packets"] == n
+
+
+def egg_settings(x=0.3):
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 41, 30, 17
+    st.grid.xmax = st.grid.ymax = st.grid.zmax = 4.0
+    st.source.position = (x, 0.2, 3.9)
+    return st
+
+
+def rigid_scene():
+    opt = S.mono(10.0, 0.1, 0.9, 1.38)
+    t = S.invert(S.rotate_y(30.0)) @ S.invert(S.translate((0.1, 0.2, 0.3)))
+    return [S.torus(0.3, 0.1, opt, 1, transform=t), S.cylinder((-.5, -.5, 0), (.5, -.5, .2), 0.1, opt, 2),
+            S.segment((-.5, .7, 0), (.5, .7, .2), opt, 3), S.box((0.3, 0.2, 0.5), opt, 4, transform=t),
+            S.box((2.0, 2.0, 2.0), S.mono(1.0, 0.1, 0.8, 1.33), 5), S.box((2.002, 2.002, 2.002), P.AMBIENT, 6)]
+
+
+def scene_and_settings(name):
+    if name == "egg":
+        return P.setup_egg(), egg_settings()
+    if name == "rigid":
+        st = P.benchmark_settings("box_slab")
+        st.grid.nxg, st.grid.nyg, st.grid.nzg = 30, 21, 17
+        return rigid_scene(), st
+    st = P.benchmark_settings(name)
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 40, 33, 50
+    return P.setup_simulation(st), st
+
+
+def same_histories(a, b):
+    for k in COUNT_KEYS:
+        assert a.stats[k] == b.stats[k], (k, a.stats[k], b.stats[k])
+    # the same lengths summed in another order: FP64 rounding of up to ~1e6 adds
+    assert np.allclose(a.jmean, b.jmean, rtol=1e-9, atol=1e-12 * b.jmean.max())
+
+
+SCENES = ["egg", "rigid", "sphere_water", "layered_vessels"]
+
+
+@pytest.mark.parametrize("kernel", ["pathlength", "weight", "test"])
+@pytest.mark.parametrize("name", SCENES)
+def test_fp32_histories_do_not_depend_on_where_the_scene_lies(gpu, name, kernel):
+    """Parameter block and device memory, cache on and off: every inlined copy of a
+    region's value rounds alike, so FP32 histories are the same."""
+    arr, st = scene_and_settings(name)
+    out = []
+    for memory, cache in ((0, 1), (0, 2), (1, 1), (1, 2)):
+        with gpu.Transport(arr, st, kernel=kernel, scene_memory=memory, nearest_cache=cache, timeout_ms=20000) as tr:
+            out.append(tr.run(20000, 3))
+    for r in out[1:]:
+        same_histories(r, out[0])
+
+
+@pytest.mark.parametrize("kernel", ["pathlength", "weight"])
+@pytest.mark.parametrize("name", SCENES)
+def test_second_moment_on_the_cache_follows_full_sweeps(gpu, name, kernel):
+    arr, st = scene_and_settings(name)
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(arr, st, kernel=kernel, nearest_cache=cache, variance=True, timeout_ms=20000) as tr:
+            out.append(tr.run_moments(20000, 3))
+    same_histories(*out)
+    a, b = out[0].jmean2, out[1].jmean2
+    # each packet adds its FP32 lengths in the order of its history, on and off the cache;
+    # the squares are summed in FP64
+    assert np.allclose(a, b, rtol=1e-9, atol=1e-12 * b.max())
+
+
+@pytest.mark.parametrize("name", ["box_slab", "layered_vessels"])
+def test_batch_follows_full_sweeps(gpu, name):
+    arr, st = scene_and_settings(name)
+    n, seeds = [9001, 300], [5, 6]
+    flat = S.FlatScene(arr)
+    optics = np.array([[(o.mus, o.mua, o.hgg, o.n) for o in flat.optics()]] * 2)
+    optics[1, :, 0] *= 0.5
+    with gpu.Batch(flat, st, 2, optics=optics) as b:
+        jm, _, per, _ = b.run(n, seeds)
+    for i in range(2):
+        own = [e for e in arr]
+        for e, o in zip(own, optics[i]):
+            e.opt = S.mono(*o)
+        with gpu.Transport(own, st, nearest_cache=2, timeout_ms=20000) as tr:
+            r = tr.run(n[i], seeds[i])
+        for k in ("packets", "rng_draws", "nscatt"):
+            assert per[i][k] == r.stats[k], (i, k, per[i][k], r.stats[k])
+        assert np.allclose(jm[i], r.jmean, rtol=1e-9, atol=1e-12 * r.jmean.max())
+
+
+@pytest.mark.parametrize("name", ["egg", "sphere_water", "layered_vessels"])
+def test_adjoint_on_the_cache_follows_full_sweeps(gpu, name):
+    """Random voxel weights, so that a step weighted by another cell than its own shows."""
+    import torch
+    arr, st = scene_and_settings(name)
+    nx, ny, nz = st.grid.nxg, st.grid.nyg, st.grid.nzg
+    w = torch.rand(nx * ny * nz, generator=torch.Generator().manual_seed(1), dtype=torch.float32).cuda()
+    groups = np.arange(len(arr)) % 4
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(arr, st, nearest_cache=cache, timeout_ms=20000) as tr:
+            out.append(tr.adjoint(20000, 3, w.data_ptr(), None, groups, 4))
+    (ga, sa), (gb, sb) = out
+    for k in COUNT_KEYS:
+        assert sa[k] == sb[k], (k, sa[k], sb[k])
+    # FP32 sums per thread of some hundred terms (2^-24 each), of both signs and up to a
+    # hundred times their sum; the packets' places on the threads differ from run to run
+    assert np.all(np.abs(ga - gb) <= 1e-3 * np.abs(gb).max(axis=1, keepdims=True)), (ga, gb)
