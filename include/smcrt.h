@@ -174,9 +174,10 @@ enum smcrt_kernel_kind {
 };
 enum smcrt_precision { SMCRT_FP32 = 0, SMCRT_FP64 = 1 };
 /* Order of the action groups in the transport kernel's per-round sorted packet
- * list (smcrt_options.group_order).  The FP64 near-surface sweeps come first and
- * the sweeps second in both; the warps take chunks of the list from its head, so
- * the last group's chunks end each round.  The order changes only the speed. */
+ * list (smcrt_options.group_order).  Both begin with the FP64 near-surface sweeps,
+ * the short steps taken in registers, the sweeps over all regions and the sweeps over
+ * the nearest ones; the warps take chunks of the list from its head, so the last
+ * group's chunks end each round.  The order changes only the speed. */
 enum smcrt_group_order {
     SMCRT_ORDER_WALK_LAST = 1,     /* ..., interactions, voxel walks, launches */
     SMCRT_ORDER_INTERACT_LAST = 2  /* ..., voxel walks, interactions, launches */

@@ -397,10 +397,11 @@ void fill_params(Params<R>* P, const smcrt_scene* scene, const smcrt_grid* grid,
     P->near_band = (R)near_band((double)P->eps, *grid);
     // the nearest-region cache: on wherever every region is 1-Lipschitz, unless
     // switched off (smcrt_autotune times both)
-    const bool allowed = cache_policy(scene, grid, (int)sizeof(R), &P->cache_margin);
+    double margin = 0;
+    const bool allowed = cache_policy(scene, grid, (int)sizeof(R), &margin);
     const int want = o ? o->nearest_cache : 0;
     P->cache_ok = allowed && want != 2 ? 1 : 0;
-    P->cache_margin_f = std::nextafter((float)P->cache_margin, INFINITY);
+    P->cache_margin = std::nextafter((float)margin, INFINITY);
     P->group_order = group_order_table(o ? o->group_order : 0);
     P->normal_h = (o && o->normal_h > 0) ? o->normal_h : 1e-6;
     P->instance = o ? o->instance : 0u;

@@ -42,9 +42,9 @@ template <class R> __host__ __device__ __forceinline__ V3<R> operator*(V3<R> a, 
 template <class R> __host__ __device__ __forceinline__ V3<R> operator*(R s, V3<R> a) { return {s * a.x, s * a.y, s * a.z}; }
 template <class R> __device__ __forceinline__ R dot3(V3<R> a, V3<R> b) { return (a.x * b.x) + (a.y * b.y) + (a.z * b.z); }
 template <class R> __device__ __forceinline__ R len3(V3<R> a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
-// Larger and smaller of two values; x where only c is a number's bound (a NaN x
-// gives c, as fmax does).  In FP64 a compare and two selects: fmax and fmin on
-// doubles are several instructions more.
+// Larger and smaller of x and a number c; a NaN x gives c, as fmax and fmin do.  In
+// FP64 a compare and a select: fmax and fmin on doubles, which also look for a NaN
+// c, are several instructions more.
 __device__ __forceinline__ float max_r(float x, float c) { return fmaxf(x, c); }
 __device__ __forceinline__ float min_r(float x, float c) { return fminf(x, c); }
 __device__ __forceinline__ double max_r(double x, double c) { return x > c ? x : c; }
@@ -663,8 +663,7 @@ struct Params {
     // nearest-region cache: allowed (every region 1-Lipschitz) and the rounding
     // margin of its test (FP32 transport: the FP32 sweeps' margin for both sweeps)
     int cache_ok;
-    double cache_margin;
-    float cache_margin_f;  // rounded up
+    float cache_margin;  // rounded up
     // sort group of each action, one nibble per action (the round's list order)
     unsigned long long group_order;
     // shared-memory fluence privatisation (FP32 plain launches): a sub-box of

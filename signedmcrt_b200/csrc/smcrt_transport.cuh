@@ -326,7 +326,17 @@ constexpr bool kNearestCache = SMCRT_NEAREST_CACHE != 0;
 constexpr bool kCacheTop = SMCRT_CACHE_TOP != 0;
 
 // Steps of one crawl (crawl_steps): the fewest lanes of a warp that go on, and the
-// most steps, in the rounds and in drain mode.
+// most steps, in the rounds and in drain mode.  Few lanes or many steps hold up the
+// warp's other packets, many lanes or few steps send more packets through the slots.
+// Ms for box_slab (1e6 packets) / sphere_water (4e6) / layered_vessels (2e6) /
+// sphere_scene (40 spheres, 2e4):
+//   16 lanes, 8 and 64 steps  15.7 / 69.7 / 41.8 / 143
+//   8 lanes                   15.4 / 68.3 / 41.0 / 143
+//   24 lanes                  15.8 / 68.5 / 42.0 / 143
+//   4 steps                   15.7 / 68.6 / 39.3 / 143
+//   16 steps                  15.7 / 70.1 / 44.7 / 143
+//   16 steps in drain mode    16.1 / 69.3 / 41.4 / 153
+//   256 steps in drain mode   15.6 / 69.5 / 41.6 / 141
 #ifndef SMCRT_CRAWL_MIN
 #define SMCRT_CRAWL_MIN 16
 #endif
@@ -337,7 +347,8 @@ constexpr bool kCacheTop = SMCRT_CACHE_TOP != 0;
 #define SMCRT_DRAIN_CRAWL 64
 #endif
 // A warp with at least this many lanes that need a sweep over all regions takes it
-// at once; fewer wait for the group of such sweeps.
+// at once; fewer wait for the group of such sweeps.  10 lanes instead of 20: 15.9 / 73.5
+// / 42.3 ms on the first three above, 28 lanes: 15.5 / 69.5 / 40.6.
 #ifndef SMCRT_FULL_MIN
 #define SMCRT_FULL_MIN 20
 #endif
@@ -394,11 +405,13 @@ struct Flight {
     };
 };
 
-// A move of f.dsdf: off the clearance, onto the bound on |d_k|.
+// Whether the kept regions alone decide at the current position: every other
+// region's |d| is above theirs by more than the rounding margin.
 template <class R>
 __device__ __forceinline__ bool cache_holds(const Params<R>& P, const Flight<R>& f) {
-    return __fadd_ru(f.dkup, P.cache_margin_f) < f.clear;
+    return __fadd_ru(f.dkup, P.cache_margin) < f.clear;
 }
+// A move of f.dsdf: off the clearance, onto the bound on |d_k|.
 template <class R>
 __device__ __forceinline__ void cache_move(Flight<R>& f) {
     f.clear = __fsub_rd(f.clear, float_ru(f.dsdf));
@@ -410,7 +423,7 @@ __device__ __forceinline__ void cache_move(Flight<R>& f) {
 // -1: none), and the launch layer (kernelsMod.f90:275-280: innermost containing
 // region).  For the nearest-region cache also the three regions of least |d|, each
 // as one word that orders by |d|: a lower bound on |d| as the bits of a float whose
-// last kBits bits are the region and whether it contains the point.
+// last KeyBits bits are the region and whether it contains the point.
 template <class T>
 struct SweepOut {
     T mna;
@@ -687,7 +700,7 @@ __device__ __forceinline__ int cell_index(const GridT<R>& g, const Flight<R>& f)
 // the lanes of a warp share one face-spacing division and one code path a segment,
 // and the packet's move after its last segment is made once, after the loop.  The
 // walk took a fifth of the transport's issue slots; with first_face this measured
-// sphere_water 88.7 -> 85.4 ms (4e6 packets), box_slab 15.0 -> 13.8 ms (1e6).
+// sphere_water 88.7 -> 85.4 ms (4e6 packets), box_slab 21.5 -> 20.2 ms (1e6).
 // (ADJ: the adjoint's track terms instead of the fluence tally; on leaving the
 // grid the rest of the step, untallied, still counts for survival.)
 template <class R, bool BATCH, bool ADJ, bool VAR>
@@ -1405,8 +1418,8 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
 // two states (a voxel walk in progress; a crossing sweep pending) and is stored
 // as raw 32-bit words.
 // Sort groups of the actions a packet can wait in between rounds, in list
-// order: FP64 near-surface sweep, sweep (or a pending crossing), then walk,
-// interact and retire/launch in the order of the launch's group_order.  Each
+// order: FP64 near-surface sweep, crawl, sweep over all regions, sweep over the kept
+// ones, then walk, interact and retire/launch in the order of the launch's group_order.  Each
 // warp's first chunk is fixed (warp w, chunk w), so the costly FP64 chunks at
 // the head of the list go to different warps; the rest of the list goes to
 // whichever warp finishes first, so the last group's chunks end each round.
@@ -1613,7 +1626,8 @@ __host__ __device__ constexpr int bins_room() {
 // injected streams.
 //
 // A CTA holds SlotTraits::n packets in shared memory.  Each round it counting-sorts
-// its live slots by their next action (warp ballots, stable in slot order), then
+// its live slots by their next action (in slot order within a warp's slots, the
+// warps of a group in the order of their shared adds), then
 // the warps take 32-item chunks of the sorted list, run one pass of each packet's
 // state machine and write the packets back.  A warp therefore works on 32
 // packets that start the pass with the same action, whatever mix of actions the
@@ -1666,8 +1680,8 @@ __global__ void __launch_bounds__(kBlock, SMCRT_MIN_BLOCKS) transport_kernel(con
     unsigned char* const vbase = VAR ? P.var_tab + (size_t)blockIdx.x * NS * kVarSlotBytes : nullptr;
     const unsigned lt = (1u << lane) - 1u;
     // ---- rounds: each round counting-sorts the live slots by action (warp
-    // ballots and a per-warp scan, stable in slot order) and the warps take
-    // 32-item chunks of the sorted list; three CTA barriers a round
+    // ballots, one shared add per warp and group, a scan of the groups) and the
+    // warps take 32-item chunks of the sorted list; three CTA barriers a round
     constexpr int Q = L::per_thread;
     constexpr int NW = kBlock / 32;
     // slots per group, of this round and (cleared) of the next
