@@ -98,6 +98,7 @@ void fill_grid(GridT<R>& g, const smcrt_grid& s) {
     g.sx = (R)s.nxg / ((R)2 * (R)s.xmax);
     g.sy = (R)s.nyg / ((R)2 * (R)s.ymax);
     g.sz = (R)s.nzg / ((R)2 * (R)s.zmax);
+    g.inset = (R)(std::max(s.xmax, std::max(s.ymax, s.zmax)) * 0x1p-31);
     g.xmax_d = s.xmax;
     g.ymax_d = s.ymax;
     g.zmax_d = s.zmax;

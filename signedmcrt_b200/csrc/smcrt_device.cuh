@@ -619,6 +619,7 @@ template <class R>
 struct GridT {
     int nx, ny, nz, pad;
     R xmax, ymax, zmax;
+    R inset;            // 2^-31 of the largest half size: crawls end this far before a voxel face
     R vx, vy, vz;       // voxel sizes 2*max/n
     R sx, sy, sz;       // n/(2*max) as written: n * p / (2 * max)
     double xmax_d, ymax_d, zmax_d;  // exact half sizes (grid-exit test on FP64 positions)

@@ -695,16 +695,17 @@ __device__ __forceinline__ int cell_index(const GridT<R>& g, const Flight<R>& f)
     return (f.w.ci - 1) + g.nx * ((f.w.cj - 1) + g.ny * (f.w.ck - 1));
 }
 
-// Voxel segments of the current step, at most SMCRT_WALK_SEGMENTS; returns true when
-// the step's walk is over.  The axis of the nearest face is picked by selects, so
-// the lanes of a warp share one face-spacing division and one code path a segment,
+// Voxel segments of the current step, at most SMCRT_WALK_SEGMENTS; returns whether
+// the step's walk goes on, or where it ended.  The axis of the nearest face is picked
+// by selects, so the lanes of a warp share one face-spacing division and one code path a segment,
 // and the packet's move after its last segment is made once, after the loop.  The
 // walk took a fifth of the transport's issue slots; with first_face this measured
 // sphere_water 88.7 -> 85.4 ms (4e6 packets), box_slab 21.5 -> 20.2 ms (1e6).
 // (ADJ: the adjoint's track terms instead of the fluence tally; on leaving the
 // grid the rest of the step, untallied, still counts for survival.)
+enum Walk : int { WALK_ON = 0, WALK_ENDS_HERE, WALK_ENDS_BEYOND };  // in the call's first cell, or a later one
 template <class R, bool BATCH, bool ADJ, bool VAR>
-__device__ __forceinline__ bool walk_segments(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, float* acc,
+__device__ __forceinline__ Walk walk_segments(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, float* acc,
                                               unsigned char* vt, unsigned long long* priv) {
     const GridT<R>& g = P.grid;
     const V3<R>& d = pk.dir;
@@ -718,7 +719,7 @@ __device__ __forceinline__ bool walk_segments(const Params<R>& P, Pk<R>& pk, Fli
         if (ADJ) adj_track(P, pk, acc, (float)len, P.adj_w[idx]);
         else tally_add<R, BATCH>(P, pk.inst, f.w.ci, f.w.cj, f.w.ck, idx, (double)len, priv);
         if (VAR) var_add(vt, P.jmean2, idx, (float)len, c);
-        if (stay) return true;
+        if (stay) return k == 0 ? WALK_ENDS_HERE : WALK_ENDS_BEYOND;
         f.w.td = tm;
         const bool bx = tm == f.w.tx, by = !bx && tm == f.w.ty;
         const R dc = bx ? d.x : by ? d.y : d.z;
@@ -740,10 +741,10 @@ __device__ __forceinline__ bool walk_segments(const Params<R>& P, Pk<R>& pk, Fli
         if (cell < 1 || cell > n) {
             pk.tflag = true;
             if (ADJ) adj_track(P, pk, acc, (float)(f.dsdf - tm), 0.0f);
-            return true;
+            return WALK_ENDS_BEYOND;
         }
     }
-    return false;
+    return WALK_ON;
 }
 
 // The end of a flight (inttau2.f90:188-209): grid-exit test, then interact or retire.
@@ -868,27 +869,27 @@ __device__ __forceinline__ int step_or_skip(const Params<R>& P, Pk<R>& pk, Fligh
 // The action of a packet that goes on with a tracing step: a crawl where the next
 // steps are known to be short (near a surface, or shorter than the way to the
 // nearest voxel face: at most dkup), else a sweep over the kept regions or all.
+// here: the walk ended in the cell its last call began in.
 template <class R>
-__device__ __forceinline__ int next_step(const Params<R>& P, const Pk<R>& pk, Flight<R>& f) {
+__device__ __forceinline__ int next_step(const Params<R>& P, const Pk<R>& pk, Flight<R>& f, bool here) {
     f.mode = S_STEP;
     if (!kNearestCache || !f.cache || !cache_holds(P, f))
         return sizeof(R) == 4 && f.near ? A_PRECISE : A_FULL;
     if (pk.tflag) return sizeof(R) == 4 && f.near ? A_PRECISE : A_SWEEP;
     const R tm = fmin(f.w.tx, fmin(f.w.ty, f.w.tz));
-    f.room = f.w.td == (R)0 ? (tm - f.dsdf) - (R)1e-6 * tm : (R)-1;
-    return f.near || (R)f.dkup < f.room ? A_CRAWL : A_SWEEP;
+    // Known: less 2^-16 of the way to the face, which is inside the inset unless the way
+    // is short or the direction almost along a face.
+    const R lim = tm - (R)0x1p-16 * tm;
+    const bool known = here && f.w.td == (R)0;
+    f.room = known ? lim - f.dsdf : (R)-1;
+    const int act = f.near || (R)f.dkup < f.room ? A_CRAWL : A_SWEEP;
+    if ((R)0x1p-16 * tm * fmin(fabs(pk.dir.x), fmin(fabs(pk.dir.y), fabs(pk.dir.z))) < P.grid.inset) f.room = (R)-1;
+    return act;
 }
 
-// What a move leaves of a crawl's room, rounded down, and 2^-24 of the room less
-// for the rounding of the position (half an ulp on each axis a step).  One
-// multiply-add, as the plain difference was one add; it ends a crawl of n steps by
-// at most n 2^-24 of the voxel early, and the general path's next step renews it.
-__device__ __forceinline__ float room_less(float room, float step) {
-    return __fmaf_rd(room, 1.0f - 0x1p-24f, -step);
-}
-__device__ __forceinline__ double room_less(double room, double step) {
-    return __fma_rd(room, 1.0 - 0x1p-24, -step);
-}
+// What a move leaves of a crawl's room, rounded down.
+__device__ __forceinline__ float room_less(float room, float step) { return __fsub_rd(room, step); }
+__device__ __forceinline__ double room_less(double room, double step) { return __dsub_rd(room, step); }
 
 // Sphere-tracing steps on the nearest-region cache inside one voxel, in registers.
 //
@@ -903,16 +904,18 @@ __device__ __forceinline__ double room_less(double room, double step) {
 // voxel face ahead, a region left, the cache no longer valid) leaves before it,
 // and the general path takes that step in its next pass.
 //
-// f.room: a lower bound on the distance along the direction to the nearest voxel
-// face, known from a walk that ended in the cell its step began in (td == 0: the
-// cell and the face distances are those of that step's start, and later positions
-// only move away from the faces behind), less 1e-6 of the face distance for the
-// rounding of the face distances.  Each step's move is taken off by room_less, which
-// rounds down: a packet along a wall makes up to millions of equal steps in one
-// voxel, and a difference rounded to nearest errs the same way at every one (up to
-// 1% of a 0.4 cm voxel at 3e-7 cm from the wall).  A step shorter than the room stays
-// in the cell in the general path too.  Negative: not known, found here from the
-// position as start_step finds it.
+// f.room: a lower bound on the way along the direction to grid.inset before the
+// nearest voxel face.  A step shorter than that stays in the cell in the general path
+// too, however they round: the inset covers the coordinate a step's cell is formed
+// from, whose rounding grows by half an ulp a step (FP64, 2^21 steps at most), and a
+// relative margin covers the face distances and the FP32 steps.  Each step's move is
+// taken off by room_less, which rounds down: a packet along a wall makes up to millions
+// of equal steps in one voxel, and a difference rounded to nearest errs the same way at
+// every one (up to 1% of a 0.4 cm voxel at 3e-7 cm from the wall).
+// Known from a walk that ended in the cell its step began in (next_step; later
+// positions only move away from the faces behind).  A walk that crossed a face, even at
+// its very start on the face, tells nothing of the cell that the next step's position
+// rounds to: negative, found here from the position as start_step finds it.
 template <class R, bool BATCH, bool ADJ, bool MODS, bool BIG, bool VAR>
 __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Flight<R>& f, Cnt& c, int& act, float* acc,
                                             unsigned char* vt, unsigned long long* priv, int crawl_min,
@@ -930,9 +933,12 @@ __device__ __forceinline__ void crawl_steps(const Params<R>& P, Pk<R>& pk, Fligh
         if (f.w.ci < 1 || f.w.ci > g.nx || f.w.cj < 1 || f.w.cj > g.ny || f.w.ck < 1 || f.w.ck > g.nz) {
             f.room = (R)0;  // outside the grid: the general path
         } else {
-            const R tm = fmin(first_face<R>(f.w.ci, g.vx_d, ox, pk.dir.x),
-                              fmin(first_face<R>(f.w.cj, g.vy_d, oy, pk.dir.y),
-                                   first_face<R>(f.w.ck, g.vz_d, oz, pk.dir.z)));
+            const V3<R>& d = pk.dir;
+            auto ahead = [&](int cell, double v, double o, R dc) {
+                return first_face<R>(cell, v, o + (double)copysign(g.inset, dc), dc);
+            };
+            const R tm = fmin(ahead(f.w.ci, g.vx_d, ox, d.x),
+                              fmin(ahead(f.w.cj, g.vy_d, oy, d.y), ahead(f.w.ck, g.vz_d, oz, d.z)));
             f.room = tm - (R)1e-6 * tm;
         }
     }
@@ -1400,14 +1406,15 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
     }
     // ---- walk voxel segments: at most SMCRT_WALK_SEGMENTS per lane per
     // iteration, so one long walk does not hold up the other lanes' actions
-    if (act == A_WALK && walk_segments<R, BATCH, ADJ, VAR>(P, pk, f, c, acc, vt, priv)) {
+    const Walk walk = act == A_WALK ? walk_segments<R, BATCH, ADJ, VAR>(P, pk, f, c, acc, vt, priv) : WALK_ON;
+    if (walk != WALK_ON) {
         pk.pos = advance(pk.pos, f.dsdf, pk.dir);
         cache_move(f);
         if (f.last) {
             act = end_flight(P, pk);  // taurun >= tau ends the flight (:100)
         } else {
             f.mode = S_STEP;
-            act = next_step(P, pk, f);
+            act = next_step(P, pk, f, walk == WALK_ENDS_HERE);
         }
     }
 }

@@ -101,6 +101,27 @@ def test_long_crawls_end_at_the_voxel_face(gpu, nz, d, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("dirx", [-1.8e-16, 1.8e-16, -1e-12, -1e-9, 1e-6])
+@pytest.mark.parametrize("x,nx", [(0.0, 4), (-1 / 3, 6), (-1 / 3 + 1e-12, 6)])
+def test_crawls_along_a_voxel_face(gpu, x, nx, dirx, precision):
+    """A beam on a voxel face, or a rounding beside it, turned from it by as little: the cells
+    are those that every step's rounded position lies in."""
+    y = float(np.float32(0.9))
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = nx, 3, 5
+    st.source.position, st.source.direction = (x, y, 1.0 - 1e-5), (dirx, 0.0, -1.0)
+    arr = [S.box((2.0, 2.0 * (y + 3e-5), 2.0), S.mono(0.0, 0.0, 0.0, 1.0), 1)]
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(arr, st, precision=precision, nearest_cache=cache, timeout_ms=60000) as tr:
+            out.append(tr.run(2, 5))
+    on, off = out
+    for k in COUNT_KEYS:
+        assert on.stats[k] == off.stats[k], (k, on.stats[k], off.stats[k])
+    assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
 @pytest.mark.parametrize("n", [1, 11000])
 def test_time_limit_in_launches_of_few_packets(gpu, n, precision):
     """The time limit ends a launch whose packets (one to 75 a CTA, up to four a warp)
