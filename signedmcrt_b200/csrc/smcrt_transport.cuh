@@ -1294,6 +1294,10 @@ __device__ __forceinline__ void transport_pass(const Params<R>& P, const Buffers
                     c.sdf += N;
                 }
                 f.steps = 0;
+                // a direction that is not finite (refracted at a normal of 0/0, where a
+                // region's four values are alike) takes the position with it, and no bound
+                // on a region's value holds there: full sweeps
+                if (kNearestCache && !(fabs(pk.dir.x + pk.dir.y + pk.dir.z) < (R)INFINITY)) f.cache = false;
                 // d == eps (reachable on the FP32 coordinate grid) counts as on the
                 // surface, like the reflected packets the reference kills here
                 if (mna <= eps) {

@@ -247,3 +247,47 @@ def test_adjoint_on_the_cache_follows_full_sweeps(gpu, name):
     # FP32 sums per thread of some hundred terms (2^-24 each), of both signs and up to a
     # hundred times their sum; the packets' places on the threads differ from run to run
     assert np.all(np.abs(ga - gb) <= 1e-3 * np.abs(gb).max(axis=1, keepdims=True)), (ga, gb)
+
+
+def plateau_scene(kind):
+    """Overlapping regions with a box revolved off its plane, whose values are one constant
+    deep inside: a crossing resolved there has no normal (0 / 0)."""
+    def at(*t):
+        m = S.identity()
+        m[3, :3] = t
+        return m
+    if kind == "beam at the rim":
+        return [S.cylinder((0, 0, -.3), (0, .1, .4), .2, S.mono(.5, 0., .5, 1.5), 1, transform=at(.25, .25, .25)),
+                S.box((.5, 1.25, .625), S.mono(.5, 1., .9, 1.33), 2,
+                      transform=at(0.3140462012492589, -0.21184131052779065, -0.4987951372882876)),
+                S.revolution(S.box((1.25, .875, .875), S.mono(20., 0., .9, 1.), 3,
+                                   transform=at(-0.41726337545446734, -0.48435662718498895, -0.40519797866702933)), .3),
+                S.box((1.8, 1.8, 1.8), S.mono(0., 0., .5, 1.33), 4)], (0.8397171426642697, 0.8266132134794663, 0.9)
+    return [S.sphere(.4, S.mono(5., 1., 0., 1.5), 1, transform=at(.5, .5, 0.)),
+            S.box((1.25, .75, .75), S.mono(5., 1., .5, 1.), 2, transform=at(-.5, -.25, -.5)),
+            S.torus(.4, .15, S.mono(.5, 1., .9, 1.33), 3, transform=at(0., .25, .5)),
+            S.revolution(S.box((1.25, 1.125, .875), S.mono(20., .05, .5, 1.33), 4, transform=at(.5, .25, -.25)), .3),
+            S.box((2., 2., 2.), S.mono(5., 0., .5, 1.33), 5), S.box((2.002, 2.002, 2.002), P.AMBIENT, 6)], (0., 0., .5)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("memory", [0, 1])
+@pytest.mark.parametrize("kernel", ["pathlength", "weight", "test"])
+@pytest.mark.parametrize("kind", ["beam at the rim", "beam at the axis"])
+def test_directions_that_are_not_numbers_leave_the_cache(gpu, kind, kernel, memory, precision):
+    """A packet refracted at a normal of 0 / 0 has no position after its next step, and no
+    bound of the cache holds there: full sweeps end it, with the cache on and off."""
+    arr, pos = plateau_scene(kind)
+    st = P.benchmark_settings("box_slab")
+    st.grid.nxg, st.grid.nyg, st.grid.nzg = 15, 37, 17
+    st.source.position = pos
+    out = []
+    for cache in (1, 2):
+        with gpu.Transport(arr, st, kernel=kernel, precision=precision, scene_memory=memory, nearest_cache=cache,
+                           max_trace_steps=20000, timeout_ms=20000) as tr:
+            out.append(tr.run(700, 28377))
+    on, off = out
+    for k in COUNT_KEYS:
+        assert on.stats[k] == off.stats[k], (k, on.stats[k], off.stats[k])
+    assert on.stats["kills_error"] == off.stats["kills_error"]
+    assert np.allclose(on.jmean, off.jmean, rtol=1e-9, atol=1e-12 * off.jmean.max())
